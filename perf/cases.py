@@ -3,7 +3,8 @@
 ``listed()`` names the cases, ``draw(rng)`` gives one more of the same ranges, ``prepare(case, seed)`` builds what a
 program holds before the call (sharded model, optimizer, token batch, weights), ``run(state)`` is one pass through the
 public entry points and returns what it computed, ``work(case)`` the bytes and operations that the pass cannot do
-without, ``tolerance(case)`` how far another correct implementation of the same precision may be off.
+without, ``tolerance(case)`` how far another correct implementation of the same precision may be off, ``exact(case, seed)`` what
+the pass gives in 64 bits with plain torch.
 
 Kinds:
 
@@ -20,6 +21,7 @@ Kinds:
 import math
 
 import torch
+import torch.utils.checkpoint
 from torch import nn
 from torch.distributed.fsdp import MixedPrecisionPolicy
 
@@ -399,3 +401,160 @@ def tolerance(case):
         return {"rel": 1e-2, "max": 0.2} if case["optimizer"] == "mixed_muon_adamw" else {"rel": 3e-2}
     return {"eval": {"rel": 3e-2}, "moe": {"rel": 2e-2, "max": 0.7}, "attention": {"rel": 1e-2, "max": 0.3},
             "muon": {"rel": 1e-2, "max": 0.15}, "ops": {"rel": 2e-2, "max": 0.4}, "module": {"rel": 1e-2}}[kind]
+
+
+# --------------------------------------------------------------------------------------------- in 64 bits
+def _norm64(x, w, eps=1e-5):
+    return x * torch.rsqrt((x * x).mean(-1, keepdim=True) + eps) * w
+
+
+def _silu64(x):
+    return x * torch.sigmoid(x)
+
+
+def _head_attention64(q, k, v):
+    """One head's [S, 128] rows; returns the output and the log-sum-exp of the scaled causal scores."""
+    scores = q @ k.T / math.sqrt(q.shape[-1])
+    scores = scores.masked_fill(torch.ones_like(scores, dtype=torch.bool).triu_(1), -math.inf)
+    lse = torch.logsumexp(scores, -1)
+    return torch.exp(scores - lse[:, None]) @ v, lse
+
+
+def _attention64(qkv, batch, seq, heads):
+    """``qkv``: [batch * seq, 3 * heads * 128]; one head at a time, recomputed in the backward pass."""
+    parts = qkv.view(batch, seq, 3, heads, 128)
+    outs, lses = [], []
+    for b in range(batch):
+        pairs = [torch.utils.checkpoint.checkpoint(_head_attention64, *(parts[b, :, i, n] for i in range(3)), use_reentrant=False)
+                 for n in range(heads)]
+        outs.append(torch.stack([o for o, _ in pairs], 1).reshape(seq, heads * 128))
+        lses.append(torch.stack([l for _, l in pairs]))
+    return torch.cat(outs), torch.stack(lses)
+
+
+def _rope64(x, seq):
+    """``x``: [batch, seq, heads, 128], pairs (i, i + 64)."""
+    inv = 10000.0 ** (-torch.arange(0, 128, 2, device=x.device, dtype=torch.float64) / 128)
+    angle = (torch.arange(seq, device=x.device, dtype=torch.float64)[:, None] * inv)[None, :, None, :]
+    a, b = x[..., :64], x[..., 64:]
+    return torch.cat([a * angle.cos() - b * angle.sin(), b * angle.cos() + a * angle.sin()], -1)
+
+
+def _units64(units):
+    """Per unit: the flat fp32 weights and, by name, 64-bit views of their bf16 values that take gradients."""
+    flats, named = [], []
+    for u in units:
+        flat = u.flat_buffer.local_shard.detach().clone()
+        leaf = flat.to(BF16).double().requires_grad_(True)
+        flats.append((flat.double(), leaf))
+        named.append({mp.fqn: leaf[mp.offset:mp.offset + mp.numel].view(mp.shape) for mp in u.registry})
+    return flats, named
+
+
+def _llama64(case, named, tokens):
+    embed = next(n for n in named if set(n) == {"weight"})["weight"]
+    head = next(n for n in named if any("lm_head" in k for k in n))
+    blocks = [n for n in named if any("w_gate" in k for k in n)]
+    assert len(blocks) == case["layers"]
+    b, s, h = *tokens.shape, 128 * case["heads"]
+    x = embed[tokens.reshape(-1)]
+    for w in blocks:
+        xn = _norm64(x, w["attn_norm.weight"])
+        q, k, v = (xn @ w[n].T for n in ("wq.weight", "wk.weight", "wv.weight"))
+        q, k = (_rope64(t.view(b, s, -1, 128), s).reshape(b * s, h) for t in (q, k))
+        x = x + _attention64(torch.cat([q, k, v], 1), b, s, case["heads"])[0] @ w["wo.weight"].T
+        xn = _norm64(x, w["mlp_norm.weight"])
+        x = x + (_silu64(xn @ w["w_gate.weight"].T) * (xn @ w["w_up.weight"].T)) @ w["w_down.weight"].T
+    return _norm64(x, head["final_norm.weight"]) @ head["lm_head.weight"].T
+
+
+def _adamw64(flats, grads, lr=3e-4, decay=0.1, beta1=0.9, eps=1e-8):
+    """First step: both moments are the gradient's after bias correction."""
+    weights = [p * (1 - lr * decay) - lr * g / (g.abs() + eps) for (p, _), g in zip(flats, grads)]
+    return dict(weights=weights, moments=[(1 - beta1) * g for g in grads])
+
+
+def _exact_train(case, seed):
+    s = _prepare_train(case, seed)
+    flats, named = _units64(s["units"])
+    loss, grads = 0.0, None
+    for tokens, targets in s["batches"]:
+        part = nn.functional.cross_entropy(_llama64(case, named, tokens), targets.reshape(-1), ignore_index=IGNORED) / len(s["batches"])
+        got = torch.autograd.grad(part, [leaf for _, leaf in flats])
+        grads = got if grads is None else [a + b for a, b in zip(grads, got)]
+        loss = part.detach()
+    _State(s)
+    if s["muon"]:
+        return dict(loss=loss, weights=[None] * len(flats))
+    if case["clip"]:
+        norm = torch.sqrt(sum((g * g).sum() for g in grads))
+        grads = [g * torch.clamp(1.0 / (norm + 1e-6), max=1.0) for g in grads]
+    return dict(loss=loss, **_adamw64(flats, grads))
+
+
+def _exact_eval(case, seed):
+    s = _prepare_eval(case, seed)
+    with torch.no_grad():
+        out = _llama64(case, _units64(s["units"])[1], s["tokens"]).view(*s["tokens"].shape, -1)
+    _State(s)
+    return out
+
+
+def _exact_attention(case, seed):
+    s = _prepare_attention(case, seed)
+    qkv = s["qkv"].double().requires_grad_(True)
+    out, lse = _attention64(qkv, *s["shape"][:3])
+    return out.detach(), lse.detach(), torch.autograd.grad(out, qkv, s["dout"].double())[0]
+
+
+def _exact_muon(case, seed):
+    s = _prepare_muon(case, seed)
+    params, moments = [], []
+    for p in s["params"]:
+        g = p.grad.double()
+        m = 0.05 * g
+        x = 0.05 * g + 0.95 * m if case["nesterov"] else m
+        x = x / x.norm()
+        for _ in range(case["steps"]):
+            gram = x.T @ x if x.shape[0] > x.shape[1] else x @ x.T
+            poly = -4.7750 * gram + 2.0315 * gram @ gram
+            x = 3.4445 * x + (x @ poly if x.shape[0] > x.shape[1] else poly @ x)
+        params.append(p.detach().double() * (1 - 0.02 * 0.1) - 0.02 * 0.2 * math.sqrt(max(p.shape)) * x)
+        moments.append(m)
+    return params, moments
+
+
+def _exact_ops(case, seed):
+    s = _prepare_ops(case, seed)
+    w = {k: v.detach().double().requires_grad_(True) for k, v in s["w"].items()}
+    x = s["x"].detach().double().requires_grad_(True)
+    gate, up = (_norm64(x, w["norm1"]) @ w["gate_up"].T).chunk(2, -1)
+    h = (_silu64(gate) * up) @ w["down"].T + x
+    loss = nn.functional.cross_entropy(_norm64(h, w["norm2"]) @ w["head"].T, s["targets"], ignore_index=IGNORED)
+    return loss.detach(), torch.autograd.grad(loss, [x, *w.values()])
+
+
+def _exact_module(case, seed):
+    s = _prepare_module(case, seed)
+    flats, named = _units64(s["units"])
+    x = s["x"].double()
+    for w in named:
+        y = nn.functional.layer_norm(x, (case["hidden"],), w["norm.weight"], w["norm.bias"])
+        x = x + nn.functional.linear(nn.functional.gelu(nn.functional.linear(y, w["up.weight"], w["up.bias"])),
+                                     w["down.weight"], w["down.bias"])
+    loss = nn.functional.mse_loss(x, s["y"].double())
+    grads = torch.autograd.grad(loss, [leaf for _, leaf in flats])
+    _State(s)
+    return dict(loss=loss.detach(), **_adamw64(flats, grads))
+
+
+_EXACT = dict(train=_exact_train, eval=_exact_eval, attention=_exact_attention, muon=_exact_muon, ops=_exact_ops,
+              module=_exact_module)
+
+
+def exact(case, seed):
+    """``None`` where 64 bits take too long (the largest products, the longest rows) and for the mixture of experts,
+    where a rounding decides which expert a token goes to and the rest follows from that."""
+    if case["kind"] == "moe" or work(case)["flops"] > 4e13 or case.get("seq", 0) > 4096:
+        return None
+    return _EXACT[case["kind"]](case, int(seed))
