@@ -12,6 +12,8 @@ here is the counterpart of those copies; everything else replaces library calls 
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
 
 from . import lib as _lib
@@ -364,6 +366,46 @@ def muon_apply_(p: torch.Tensor, o: torch.Tensor, rows: int, cols: int, transpos
                                      p_lp.data_ptr() if p_lp is not None else None, rows, cols,
                                      int(transposed), lr, weight_decay, adjusted_lr, _stream()),
                "muon_apply")
+
+
+MUON_BATCH = 64      # matrices whose addresses fit one launch's parameters
+
+
+def _addresses(tensors: list) -> "C.Array":
+    for t in tensors:
+        if t is not None and not t.is_contiguous():
+            raise RuntimeError("Muon's matrices, gradients and momentum buffers must be contiguous")
+    return (C.c_ulonglong * len(tensors))(*[0 if t is None else t.data_ptr() for t in tensors])
+
+
+def muon_prepare(bufs: list, grads: list, mu: float, grad_scale: float, nesterov: bool, eps: float) -> torch.Tensor:
+    """Momentum, Nesterov and Frobenius scaling of same-shape matrices: ``bufs`` (fp32) are updated, the result is the
+    stacked bf16 ``[G, rows, cols]``.  ``grads``: all bf16 or all fp32."""
+    shape, n, dt = bufs[0].shape, bufs[0].numel(), grads[0].dtype
+    assert dt in (torch.bfloat16, torch.float32)
+    assert all(b.dtype == torch.float32 and b.shape == shape for b in bufs)
+    assert all(g.dtype == dt and g.shape == shape for g in grads)
+    out = torch.empty((len(bufs), *shape), dtype=torch.bfloat16, device=bufs[0].device)
+    partial = torch.empty(min(len(bufs), MUON_BATCH) * _L().mfsdp_muon_partials(1, n), dtype=torch.float32, device=out.device)
+    for i in range(0, len(bufs), MUON_BATCH):
+        b, g = bufs[i:i + MUON_BATCH], grads[i:i + MUON_BATCH]
+        _lib.check(_L().mfsdp_muon_prepare_many(_addresses(b), _addresses(g), len(b), int(dt == torch.bfloat16),
+                                                out[i].data_ptr(), partial.data_ptr(), n, mu, grad_scale, int(nesterov),
+                                                eps, _stream()), "muon_prepare_many")
+    return out
+
+
+def muon_apply_many_(ps: list, o: torch.Tensor, lps: list, lr: float, weight_decay: float, adjusted_lr: float) -> None:
+    """``p = p (1 - lr wd) - adjusted_lr o[i]`` for same-shape fp32 matrices; ``lps``: their bf16 copies or ``None``."""
+    n = ps[0].numel()
+    o = o.reshape(len(ps), n)
+    assert o.dtype == torch.bfloat16 and o.is_contiguous()
+    assert all(p.dtype == torch.float32 and p.numel() == n for p in ps)
+    assert all(t is None or (t.dtype == torch.bfloat16 and t.numel() == n) for t in lps)
+    for i in range(0, len(ps), MUON_BATCH):
+        p = ps[i:i + MUON_BATCH]
+        _lib.check(_L().mfsdp_muon_apply_many(_addresses(p), _addresses(lps[i:i + MUON_BATCH]), len(p), o[i].data_ptr(), n,
+                                              lr, weight_decay, adjusted_lr, _stream()), "muon_apply_many")
 
 
 # ------------------------------------------------------------------ copies

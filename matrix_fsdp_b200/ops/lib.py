@@ -40,6 +40,9 @@ _SIGNATURES: dict[str, list] = {
     "mfsdp_muon_momentum": [vp, vp, i32, vp, vp, i64, f32, f32, i32, vp],
     "mfsdp_muon_normalize": [vp, vp, i64, f32, vp],
     "mfsdp_muon_apply": [vp, vp, vp, i32, i32, i32, f32, f32, f32, vp],
+    "mfsdp_muon_partials": [i32, i64],
+    "mfsdp_muon_prepare_many": [vp, vp, i32, i32, vp, vp, i64, f32, f32, i32, f32, vp],
+    "mfsdp_muon_apply_many": [vp, vp, i32, vp, i64, f32, f32, f32, vp],
     "mfsdp_copy_segments": [vp, vp, vp, vp, vp, i32, i64, i32, vp],
     "mfsdp_cast_f32_bf16": [vp, vp, i64, vp],
 }
@@ -93,7 +96,7 @@ def available() -> bool:
 
 
 # kernels launched per launcher call (default 1); the counter feeds the benchmark's launch report
-_KERNELS_PER_CALL = {"rmsnorm_bwd": 2, "mfsdp_attention_bwd": 3}
+_KERNELS_PER_CALL = {"rmsnorm_bwd": 2, "muon_prepare_many": 2, "mfsdp_attention_bwd": 3}
 _LAUNCH_COUNT = [0]
 
 

@@ -245,16 +245,19 @@ class MatrixMuon(Optimizer):
             by_shape: dict[tuple, list] = {}
             for p in todo:
                 if self._kernel_path(p) and can_batch_newton_schulz(p.shape):
-                    by_shape.setdefault(tuple(p.shape), []).append(p)
+                    by_shape.setdefault((tuple(p.shape), self._grad_of(p).dtype), []).append(p)
                 else:
                     self._apply(p, self._orthogonalize([self._prepare(p, group)], group)[0], group)
-            # matrices of one shape go through Newton-Schulz together (one grouped launch per product)
-            for shape, ps in by_shape.items():
+            # matrices of one shape go through every stage together (one grouped launch per product)
+            for (shape, _), ps in by_shape.items():
                 per_chunk = max(1, MAX_BATCH_ELEMENTS // (shape[0] * shape[1]))
                 for i in range(0, len(ps), per_chunk):
                     chunk = ps[i:i + per_chunk]
-                    for p, o in zip(chunk, self._orthogonalize([self._prepare(p, group) for p in chunk], group)):
-                        self._apply(p, o, group)
+                    self.ns_matrices_done += len(chunk)
+                    x = self._prepare_many(chunk, group)
+                    ns = newton_schulz_sm100_batched if len(chunk) > 1 else newton_schulz_sm100
+                    x = ns(x if len(chunk) > 1 else x[0], group["ns_coefficients"], group["ns_steps"])
+                    self._apply_many(chunk, x, group)
         return loss
 
     def _grad_of(self, p):
@@ -271,24 +274,47 @@ class MatrixMuon(Optimizer):
     def _prepare(self, p: torch.Tensor, group: dict) -> torch.Tensor:
         """Momentum + Nesterov; returns the Newton-Schulz operand (kernel path: bf16, already divided by its
         Frobenius norm; otherwise the raw update, normalised inside the reference iteration)."""
+        if self._kernel_path(p):
+            return self._prepare_many([p], group)[0]
         st = self.state[p]
-        kernels = self._kernel_path(p)
         if "momentum_buffer" not in st:
             st["momentum_buffer"] = torch.zeros_like(p, dtype=torch.float32 if p.dtype == torch.float32 else p.dtype)
         buf, mu, g = st["momentum_buffer"], group["momentum"], self._grad_of(p)
-        if kernels:
-            from ..ops import kernels as K
-
-            u = torch.empty(p.shape, dtype=torch.bfloat16, device=p.device)
-            ss = torch.zeros(1, dtype=torch.float32, device=p.device)
-            K.muon_momentum(buf.view(-1), g.reshape(-1), u.view(-1), ss, mu, float(self.grad_scale), group["nesterov"])
-            K.muon_normalize_(u.view(-1), ss, group["eps"])
-            return u
         gf = g.to(buf.dtype)
         if self.grad_scale != 1.0:
             gf = gf * self.grad_scale
         buf.lerp_(gf, 1 - mu)
         return gf.lerp(buf, mu) if group["nesterov"] else buf
+
+    def _prepare_many(self, ps: list, group: dict) -> torch.Tensor:
+        """The kernel path of :meth:`_prepare` for matrices of one shape and gradient dtype: ``[G, rows, cols]``, the
+        normalised operands stacked as the grouped Newton-Schulz reads them."""
+        from ..ops import kernels as K
+
+        bufs = []
+        for p in ps:
+            st = self.state[p]
+            buf = st.get("momentum_buffer")
+            if buf is None:
+                buf = st["momentum_buffer"] = torch.zeros_like(p, dtype=torch.float32)
+            bufs.append(buf)
+        grads = [self._grad_of(p) for p in ps]
+        if grads[0].dtype not in (torch.float32, torch.bfloat16):
+            grads = [g.float() for g in grads]
+        return K.muon_prepare(bufs, grads, group["momentum"], float(self.grad_scale), group["nesterov"], group["eps"])
+
+    def _apply_many(self, ps: list, o: torch.Tensor, group: dict) -> None:
+        """The kernel path of :meth:`_apply` for the stacked results of matrices of one shape."""
+        from ..ops import kernels as K
+
+        lr = float(group["lr"])
+        lps = [self._low_precision_of(p) if self._low_precision_of is not None else None for p in ps]
+        K.muon_apply_many_([p.data for p in ps], o,
+                           [lp if lp is not None and lp.dtype == torch.bfloat16 else None for lp in lps],
+                           lr, group["weight_decay"], adjust_lr(lr, group["adjust_lr_fn"], ps[0].shape))
+        for p, lp in zip(ps, lps):
+            if lp is not None and lp.dtype != torch.bfloat16:
+                lp.copy_(p.data)
 
     def _orthogonalize(self, us: list, group: dict) -> list:
         """Newton-Schulz on each operand; same-shape bf16 CUDA operands go through the grouped kernels together."""
@@ -301,17 +327,12 @@ class MatrixMuon(Optimizer):
                 for u, nat in zip(us, native)]
 
     def _apply(self, p: torch.Tensor, o: torch.Tensor, group: dict) -> None:
+        if self._kernel_path(p) and o.dtype == torch.bfloat16:
+            self._apply_many([p], o, group)
+            return
         lr, wd = float(group["lr"]), group["weight_decay"]
         alr = adjust_lr(lr, group["adjust_lr_fn"], p.shape)
         lp = self._low_precision_of(p) if self._low_precision_of is not None else None
-        if self._kernel_path(p) and o.dtype == torch.bfloat16:
-            from ..ops import kernels as K
-
-            K.muon_apply_(p.data.view(-1), o.reshape(-1), p.shape[0], p.shape[1], False, lr, wd, alr,
-                          p_lp=lp.view(-1) if lp is not None and lp.dtype == torch.bfloat16 else None)
-            if lp is not None and lp.dtype != torch.bfloat16:
-                lp.copy_(p.data)
-            return
         p.data.mul_(1 - lr * wd)
         p.data.add_(o.to(p.dtype), alpha=-alr)
         if lp is not None:

@@ -153,3 +153,35 @@ def test_newton_schulz_symmetric_products_match_full_products(monkeypatch):
         assert _rel(a, b) < 2e-2
         if ab is not None:
             assert _rel(ab[0], b) < 2e-2 and _rel(ab[1], b) < 2e-2
+
+
+@pytest.mark.parametrize("gdtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("mats,rows,cols,shift", [(1, 128, 128, 0), (65, 8, 24, 0), (3, 7, 13, 0), (2, 640, 264, 1), (4, 16, 8, 4)])
+def test_muon_stages_of_many_matrices(mats, rows, cols, shift, gdtype):
+    """One and several launches, sizes below a vector, remainders, bases off the 16-byte grid.  Bounds: fp32 sums of
+    three terms (1e-6 of the operands), one bf16 rounding before and one after the scaling (2^-8 together)."""
+    from matrix_fsdp_b200.ops import kernels as K
+
+    torch.manual_seed(3)
+    n, dev = rows * cols, "cuda"
+
+    def views(dtype, scale=1.0):
+        base = (scale * torch.randn(mats, n + 8, device=dev)).to(dtype)
+        return [base.as_strided((rows, cols), (cols, 1), i * (n + 8) + shift) for i in range(mats)]
+
+    bufs, grads, ps = views(torch.float32), views(gdtype), views(torch.float32, 0.02)
+    lps = [torch.zeros(rows, cols, dtype=torch.bfloat16, device=dev) if i % 2 == 0 else None for i in range(mats)]
+    mu, scale, lr, wd, alr = 0.95, 0.5, 0.02, 0.1, 0.03
+    b0, p0 = [b.double() for b in bufs], [p.double() for p in ps]
+    out = K.muon_prepare(bufs, grads, mu, scale, True, 1e-7)
+    K.muon_apply_many_(ps, out, lps, lr, wd, alr)
+    assert out.shape == (mats, rows, cols)
+    for i in range(mats):
+        g = grads[i].double() * scale
+        b = b0[i] + (1 - mu) * (g - b0[i])
+        u = g + mu * (b - g)
+        assert _rel(bufs[i], b) < 1e-6
+        assert _rel(out[i], u / u.norm()) < 2 ** -8
+        assert _rel(ps[i], p0[i] * (1 - lr * wd) - alr * out[i].double()) < 1e-6
+        if lps[i] is not None:
+            assert torch.equal(lps[i], ps[i].bfloat16())
