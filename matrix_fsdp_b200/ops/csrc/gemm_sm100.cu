@@ -56,7 +56,8 @@ struct GemmArgs {
   int tile_m;                // rows of one work item: 128, or 256 for CTA pairs
   // Symmetric output (sym_rows > 0): every output matrix is sym_rows*128 square and equal to its own
   // transpose (X Xᵀ, polynomials of it), so only tiles that reach the diagonal or lie above it are
-  // computed; the caller mirrors the rest.  Work items enumerate exactly those tiles, row by row.
+  // computed, and the epilogue stores those above it a second time, transposed, into the mirrored place.
+  // Work items enumerate exactly those tiles, row by row.
   int sym_rows;              // tile rows (of tile_m rows) per symmetric matrix (0 = off)
   int sym_q;                 // tile width / tile_m (1 or 2)
   int sym_tiles_per_matrix;
@@ -105,6 +106,9 @@ struct TileCoord {
   int nkb;           // number of 64-wide reduce blocks
   int b_row_off;     // mode 1: offset added to B's row coordinate
   bool skip;
+  bool mirror;       // symmetric output: the tile lies above the diagonal tiles
+  int mirror_row0;   // first row of D of this tile's matrix
+  int mirror_col0;   // first column of the mirrored place inside the matrix (= the tile's first row)
 };
 
 // Tiles of tile-row i of a symmetric matrix that lie entirely below the diagonal: floor(i / q); the
@@ -115,7 +119,7 @@ __host__ __device__ __forceinline__ int sym_kept_before(int i, int tiles_n, int 
 }
 
 __device__ __forceinline__ TileCoord decode_tile(const GemmArgs& p, int tile) {
-  int tm, tn;
+  int tm, tn, sym_row = 0;
   if (p.sym_rows > 0) {
     const int mat = tile / p.sym_tiles_per_matrix;
     const int rem = tile - mat * p.sym_tiles_per_matrix;
@@ -124,6 +128,7 @@ __device__ __forceinline__ TileCoord decode_tile(const GemmArgs& p, int tile) {
       const int mid = (lo + hi + 1) >> 1;
       if (sym_kept_before(mid, p.tiles_n, p.sym_q) <= rem) lo = mid; else hi = mid - 1;
     }
+    sym_row = lo;
     tm = mat * p.sym_rows + lo;
     tn = lo / p.sym_q + (rem - sym_kept_before(lo, p.tiles_n, p.sym_q));
   } else {
@@ -161,6 +166,9 @@ __device__ __forceinline__ TileCoord decode_tile(const GemmArgs& p, int tile) {
     c.a_row_k0 = k_lo;
     c.nkb = (k_hi - k_lo + BK - 1) / BK;
   }
+  c.mirror = p.sym_rows > 0 && tn > sym_row / p.sym_q;
+  c.mirror_col0 = sym_row * p.tile_m;
+  c.mirror_row0 = c.out_row0 - c.mirror_col0;
   return c;
 }
 
@@ -168,7 +176,8 @@ template <int BN, bool A_MN, bool B_MN, bool GATHER = false, bool TWO_SM = false
 __global__ void __launch_bounds__(GATHER ? kGemmThreads + kGatherThreads : kGemmThreads, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
                          const __grid_constant__ CUtensorMap tma_b,
-                         const __grid_constant__ CUtensorMap tma_d, const GemmArgs p) {
+                         const __grid_constant__ CUtensorMap tma_d,
+                         const __grid_constant__ CUtensorMap tma_t, const GemmArgs p) {
   static_assert(!(TWO_SM && GATHER) && (!TWO_SM || BN == 256), "CTA pairs: dense 256 x 256 tiles only");
   using Cfg = GemmCfg<BN, TWO_SM>;
   // CTA pairs: `worker` indexes the pair, `cta_rank` the CTA inside it (0 = leader, issues the MMAs)
@@ -384,9 +393,14 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
       for (int ch = 0; ch < BN / 64; ++ch) {
         const int ncol0 = n0 + ch * 64;
         if (ncol0 >= p.N) break;
-        const uint32_t buf = store_cnt & 1;
+        // symmetric outputs use the second buffer for the transposed copy of the chunk
+        const uint32_t buf = p.sym_rows > 0 ? 0u : (store_cnt & 1);
         uint8_t* ebuf = epi_base + buf * kEpiBufBytes;
-        if (epi_tid == 0) tma_store_wait_read<1>();
+        uint8_t* tbuf = epi_base + kEpiBufBytes + (row_in_tile >> 6) * 8192 + (row_in_tile & 7) * 2;
+        if (epi_tid == 0) {
+          if (p.sym_rows > 0) tma_store_wait_read<0>();
+          else tma_store_wait_read<1>();
+        }
         epi_bar_sync();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -433,12 +447,26 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
             const int phys = chunk ^ (row_in_tile & 7);
             *reinterpret_cast<uint4*>(ebuf + row_in_tile * 128 + phys * 16) = o;
           }
+          if (c.mirror) {
+            // column j of the chunk becomes a row of two 64 x 64 swizzled blocks (rows 0-63 and 64-127 of the tile);
+            // a warp's 32 lanes write 64 consecutive bytes per column (no bank conflicts)
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const int phys = ((row_in_tile & 63) >> 3) ^ (j & 7);
+              *reinterpret_cast<__nv_bfloat16*>(tbuf + (h * 32 + j) * 128 + phys * 16) = __float2bfloat16_rn(v[j]);
+            }
+          }
         }
         fence_proxy_async_smem();
         epi_bar_sync();
         // (a pair's second CTA may own no rows at all at the bottom edge: nothing to store then)
         if (epi_tid == 0 && (!TWO_SM || c.m0 + pair_row < p.M)) {
           tma_store_2d(&tma_d, smem_u32(ebuf), ncol0, c.out_row0 + pair_row);
+          if (c.mirror) {
+            const uint32_t t = smem_u32(epi_base + kEpiBufBytes);
+            tma_store_2d(&tma_t, t, c.mirror_col0 + pair_row, c.mirror_row0 + ncol0);
+            tma_store_2d(&tma_t, t + 8192, c.mirror_col0 + pair_row + 64, c.mirror_row0 + ncol0);
+          }
           tma_store_commit();
         }
         ++store_cnt;
@@ -558,7 +586,7 @@ int make_tmap_bf16_2d(CUtensorMap* map, const void* base, long long rows, long l
 
 template <int BN, bool A_MN, bool B_MN, bool GATHER = false>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td,
-                       const GemmArgs& args, int grid, cudaStream_t stream) {
+                       const CUtensorMap& tt, const GemmArgs& args, int grid, cudaStream_t stream) {
   using Cfg = GemmCfg<BN>;
   static bool attr_set = false;
   auto kern = gemm_bf16_tcgen05_kernel<BN, A_MN, B_MN, GATHER>;
@@ -568,7 +596,7 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
-  kern<<<grid, GATHER ? kGemmThreads + kGatherThreads : kGemmThreads, Cfg::kSmemBytes, stream>>>(ta, tb, td, args);
+  kern<<<grid, GATHER ? kGemmThreads + kGatherThreads : kGemmThreads, Cfg::kSmemBytes, stream>>>(ta, tb, td, tt, args);
   return (int)cudaGetLastError();
 }
 
@@ -576,7 +604,7 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
 // resident at once (a GPC with an odd number of free SMs leaves one without a partner).
 template <bool A_MN, bool B_MN>
 static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td,
-                            const GemmArgs& args, int num_sms, cudaStream_t stream) {
+                            const CUtensorMap& tt, const GemmArgs& args, int num_sms, cudaStream_t stream) {
   using Cfg = GemmCfg<256, true>;
   auto kern = gemm_bf16_tcgen05_kernel<256, A_MN, B_MN, false, true>;
   static int max_pairs = -1;
@@ -604,7 +632,7 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const 
   int pairs = args.total_tiles < max_pairs ? args.total_tiles : max_pairs;
   if (pairs > num_sms / 2) pairs = num_sms / 2;
   cfg.gridDim = dim3((unsigned)(2 * pairs));
-  return (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, td, args);
+  return (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, td, tt, args);
 }
 
 // MFSDP_GEMM_2SM = 1 (default): CTA pairs whenever the problem is eligible (measured 3-14 % faster than the
@@ -729,7 +757,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* D, const void* Cin
   args.b_group_stride = (group_mode == 1) ? (b_mn_major ? K : N) : 0;
 
   // Tensor maps.
-  CUtensorMap ta, tb, td;
+  CUtensorMap ta, tb, td, tt;
   int rc;
   const long long red = (group_mode == 2) ? k_total : K;
   if (!a_mn_major) rc = make_tmap_bf16_2d(&ta, A, M, red, lda, BM, 64);
@@ -742,6 +770,9 @@ static int gemm_bf16_impl(const void* A, const void* B, void* D, const void* Cin
   const long long d_rows = (group_mode == 2) ? (long long)M * num_groups : M;
   rc = make_tmap_bf16_2d(&td, D, d_rows, N, ldd, BM, 64);
   if (rc) return rc;
+  tt = td;
+  if (symmetric) rc = make_tmap_bf16_2d(&tt, D, d_rows, N, ldd, 64, 64);
+  if (rc) return rc;
 
   int total = args.tiles_m * args.tiles_n;
   if (symmetric) {
@@ -752,17 +783,17 @@ static int gemm_bf16_impl(const void* A, const void* B, void* D, const void* Cin
   }
   args.total_tiles = total;
   if (pair) {
-    return a_mn_major ? (b_mn_major ? launch_gemm_pair<true, true>(ta, tb, td, args, num_sms, stream)
-                                    : launch_gemm_pair<true, false>(ta, tb, td, args, num_sms, stream))
-                      : (b_mn_major ? launch_gemm_pair<false, true>(ta, tb, td, args, num_sms, stream)
-                                    : launch_gemm_pair<false, false>(ta, tb, td, args, num_sms, stream));
+    return a_mn_major ? (b_mn_major ? launch_gemm_pair<true, true>(ta, tb, td, tt, args, num_sms, stream)
+                                    : launch_gemm_pair<true, false>(ta, tb, td, tt, args, num_sms, stream))
+                      : (b_mn_major ? launch_gemm_pair<false, true>(ta, tb, td, tt, args, num_sms, stream)
+                                    : launch_gemm_pair<false, false>(ta, tb, td, tt, args, num_sms, stream));
   }
   const int grid = total < num_sms ? total : num_sms;
 #define MFSDP_LAUNCH(BN_)                                                                   \
-  (a_mn_major ? (b_mn_major ? launch_gemm<BN_, true, true>(ta, tb, td, args, grid, stream)  \
-                            : launch_gemm<BN_, true, false>(ta, tb, td, args, grid, stream)) \
-              : (b_mn_major ? launch_gemm<BN_, false, true>(ta, tb, td, args, grid, stream) \
-                            : launch_gemm<BN_, false, false>(ta, tb, td, args, grid, stream)))
+  (a_mn_major ? (b_mn_major ? launch_gemm<BN_, true, true>(ta, tb, td, tt, args, grid, stream)  \
+                            : launch_gemm<BN_, true, false>(ta, tb, td, tt, args, grid, stream)) \
+              : (b_mn_major ? launch_gemm<BN_, false, true>(ta, tb, td, tt, args, grid, stream) \
+                            : launch_gemm<BN_, false, false>(ta, tb, td, tt, args, grid, stream)))
   return bn == 256 ? MFSDP_LAUNCH(256) : MFSDP_LAUNCH(128);
 #undef MFSDP_LAUNCH
 }
@@ -779,8 +810,9 @@ MFSDP_API int mfsdp_gemm_bf16(const void* A, const void* B, void* D, const void*
 
 // Same product for outputs known to be symmetric (every output matrix is N x N with N a multiple of 128:
 // M == N, or M a multiple of N in the M-grouped mode).  Only the tiles on or above the diagonal are
-// computed and written; entries below the diagonal that fall outside those tiles are left untouched, so
-// the caller follows with mfsdp_mirror_upper.
+// computed; the others are written as their transposes, from the same values.  (A second kernel that
+// mirrored finished matrices took 95 us per launch for 64 matrices of 2048 x 2048; without it the optimizer
+// step of two 2048-wide blocks went from 4.63 to 4.35 ms, the step of 64 experts in each of 2 layers from 65.5 to 64.2.)
 MFSDP_API int mfsdp_gemm_bf16_sym(const void* A, const void* B, void* D, const void* Cin, int M, int N,
                                   int K, long long lda, long long ldb, long long ldd, long long ldcin,
                                   int a_mn_major, int b_mn_major, float alpha, float beta,
@@ -789,32 +821,6 @@ MFSDP_API int mfsdp_gemm_bf16_sym(const void* A, const void* B, void* D, const v
                                   int force_bn, cudaStream_t stream) {
   return gemm_bf16_impl(A, B, D, Cin, M, N, K, lda, ldb, ldd, ldcin, a_mn_major, b_mn_major, alpha, beta, group_mode,
                         tile_group, group_offsets, num_groups, k_total, status, num_sms, force_bn, 1, stream);
-}
-
-// D[i][j] = D[j][i] for i > j, for `mats` stacked n x n matrices (n a multiple of 64), 64 x 64 blocks.
-__global__ void __launch_bounds__(256) mirror_upper_kernel(__nv_bfloat16* __restrict__ d, int n, long long ldd) {
-  __shared__ unsigned short tile[64][66];
-  const int bj = blockIdx.x, bi = blockIdx.y;
-  if (bi <= bj) return;                           // diagonal blocks were computed whole
-  unsigned short* base = reinterpret_cast<unsigned short*>(d) + (long long)blockIdx.z * n * ldd;
-  const int cp = threadIdx.x & 31, r0 = threadIdx.x >> 5;
-  for (int r = r0; r < 64; r += 8) {              // source block (bj, bi): above the diagonal
-    const unsigned v = *reinterpret_cast<const unsigned*>(base + (long long)(bj * 64 + r) * ldd + bi * 64 + 2 * cp);
-    tile[r][2 * cp] = (unsigned short)(v & 0xffffu);
-    tile[r][2 * cp + 1] = (unsigned short)(v >> 16);
-  }
-  __syncthreads();
-  for (int r = r0; r < 64; r += 8) {              // destination block (bi, bj), row r = source column r
-    const unsigned v = (unsigned)tile[2 * cp][r] | ((unsigned)tile[2 * cp + 1][r] << 16);
-    *reinterpret_cast<unsigned*>(base + (long long)(bi * 64 + r) * ldd + bj * 64 + 2 * cp) = v;
-  }
-}
-
-MFSDP_API int mfsdp_mirror_upper(void* D, int n, long long ldd, int mats, cudaStream_t stream) {
-  if (n <= 0 || (n % 64) != 0 || (ldd % 2) != 0 || mats <= 0 || ((uintptr_t)D & 3)) return -2;
-  if (n == 64) return 0;
-  mirror_upper_kernel<<<dim3(n / 64, n / 64, mats), 256, 0, stream>>>((__nv_bfloat16*)D, n, ldd);
-  return (int)cudaGetLastError();
 }
 
 // All-gather fused into the GEMM that first consumes the gathered weight:
@@ -861,6 +867,6 @@ MFSDP_API int mfsdp_gemm_bf16_ag(const void* A, const void* B, void* D, const vo
   const int total = args.tiles_m * args.tiles_n;
   args.total_tiles = total;
   const int grid = total < num_sms ? total : num_sms;
-  return bn == 256 ? launch_gemm<256, false, false, true>(ta, tb, td, args, grid, stream)
-                   : launch_gemm<128, false, false, true>(ta, tb, td, args, grid, stream);
+  return bn == 256 ? launch_gemm<256, false, false, true>(ta, tb, td, td, args, grid, stream)
+                   : launch_gemm<128, false, false, true>(ta, tb, td, td, args, grid, stream);
 }

@@ -87,7 +87,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
     ``a`` is ``[M,K]`` (or ``[K,M]`` when ``a_mn_major``); ``b`` is ``[N,K]`` (or ``[K,N]`` when
     ``b_mn_major``).  Row strides must be multiples of 8 elements, inner stride 1.
     ``symmetric``: the caller knows the result equals its transpose (M == N, a multiple of 128); only the
-    tiles on or above the diagonal are computed and the rest is mirrored (about half the tensor-core work).
+    tiles on or above the diagonal are computed, each is also stored transposed (about half the tensor-core work).
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
     assert a.dim() == 2 and b.dim() == 2 and a.stride(1) == 1 and b.stride(1) == 1
@@ -113,18 +113,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
         int(a_mn_major), int(b_mn_major), float(alpha), float(beta), 0, None, None, 0, 0,
         status_word(a.device).data_ptr(), sm_count(a.device), force_bn, _stream())
     _lib.check(rc, "mfsdp_gemm_bf16")
-    if symmetric:
-        mirror_upper_(out, 1)
     return out
-
-
-def mirror_upper_(d: torch.Tensor, mats: int = 1) -> torch.Tensor:
-    """``d``: ``mats`` square matrices stacked along dim 0 (``[mats * n, n]``); copies each matrix's upper
-    triangle onto its lower one in 64 x 64 blocks (diagonal blocks are left as they are)."""
-    n = d.shape[-1]
-    assert d.dtype == torch.bfloat16 and d.stride(-1) == 1 and d.numel() == mats * n * n and d.is_contiguous()
-    _lib.check(_L().mfsdp_mirror_upper(d.data_ptr(), n, n, mats, _stream()), "mfsdp_mirror_upper")
-    return d
 
 
 def gemm_ag(a: torch.Tensor, b: torch.Tensor, plan, *, out: torch.Tensor | None = None,
@@ -163,7 +152,7 @@ def grouped_gemm_m(a: torch.Tensor, b: torch.Tensor, tile_group: torch.Tensor, *
     ``a``: ``[Mtot, K]``; ``b``: ``[G, N, K]`` (or ``[G, K, N]`` when ``b_mn_major``); tiles whose
     group id is negative are skipped (their output rows are left untouched).  ``symmetric``: ``a`` stacks
     ``Mtot / N`` blocks of ``N`` rows whose outputs are symmetric ``N x N`` matrices (``N`` a multiple of 128);
-    tiles below the diagonal are mirrored instead of computed.  ``groups_of_256_rows``: the caller's promise that
+    tiles below the diagonal are transposes instead of computed.  ``groups_of_256_rows``: the caller's promise that
     every group has a multiple of 256 rows, which lets the two-CTA kernel (256 x 256 tiles) run.
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and b.dim() == 3
@@ -191,8 +180,6 @@ def grouped_gemm_m(a: torch.Tensor, b: torch.Tensor, tile_group: torch.Tensor, *
         float(alpha), float(beta), 1, tile_group.data_ptr(), None, G, 0,
         status_word(a.device).data_ptr(), sm_count(a.device), 2 if groups_of_256_rows and Mtot % 256 == 0 else 0, _stream())
     _lib.check(rc, "mfsdp_gemm_bf16[m-grouped]")
-    if symmetric:
-        mirror_upper_(out, Mtot // N)
     return out
 
 
@@ -216,8 +203,6 @@ def grouped_gemm_k(a: torch.Tensor, b: torch.Tensor, group_offsets: torch.Tensor
         1, 1, 1.0, 0.0, 2, None, group_offsets.data_ptr(), num_groups, Ktot,
         status_word(a.device).data_ptr(), sm_count(a.device), 0, _stream())
     _lib.check(rc, "mfsdp_gemm_bf16[k-grouped]")
-    if symmetric:
-        mirror_upper_(out.view(num_groups * M, N), num_groups)
     return out
 
 

@@ -24,7 +24,6 @@ _SIGNATURES: dict[str, list] = {
                         i32, vp, vp, i32, i64, vp, i32, i32, vp],
     "mfsdp_gemm_bf16_sym": [vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, i64, i32, i32, f32, f32,
                             i32, vp, vp, i32, i64, vp, i32, i32, vp],
-    "mfsdp_mirror_upper": [vp, i32, i64, i32, vp],
     "mfsdp_gemm_bf16_ag": [vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, f32, f32, vp, vp, vp, vp, i32, vp, vp, vp, i32,
                            i32, C.c_ulonglong, vp, i32, vp],
     "mfsdp_rmsnorm_fwd": [vp, vp, vp, vp, i64, i32, f32, vp],

@@ -11,7 +11,7 @@ On CUDA each Newton-Schulz product runs on the tcgen05 GEMM with the polynomial 
 the epilogue (``alpha * acc + beta * C``), so an iteration is three kernels with no separate
 axpy, and tall matrices are handled by switching operand majors instead of transposing.  The Gram
 matrix and its polynomial are symmetric: their GEMMs compute only the tiles that reach the diagonal
-or lie above it and a small block-transpose kernel mirrors the rest (two of the three products of an
+or lie above it and store the latter twice, once transposed (two of the three products of an
 iteration do about half the tensor-core work).  The
 element-wise stages (momentum/Nesterov + Frobenius norm, scaling, parameter update + bf16 emit)
 are single fused kernels.  The reference delegates all of this to ``torch.optim.Muon``
@@ -31,7 +31,7 @@ DEFAULT_MUON_ADJUST_LR_FN = "match_rms_adamw"
 EPS = 1e-7
 MAX_BATCH_ELEMENTS = 1 << 28      # elements of one stacked Newton-Schulz operand (512 MB of bf16)
 SHARE_WINDOW_ELEMENTS = 1 << 29   # elements exchanged per all-reduce when replicas share Newton-Schulz (1 GB of bf16)
-# X Xᵀ and b A + c A A are symmetric: compute the tiles on or above the diagonal, mirror the rest
+# X Xᵀ and b A + c A A are symmetric: compute the tiles on or above the diagonal, store them twice
 SYMMETRIC_PRODUCTS = os.environ.get("MFSDP_MUON_SYMMETRIC", "1") != "0"
 
 
@@ -61,10 +61,9 @@ def newton_schulz_reference(u: torch.Tensor, coefficients=DEFAULT_NS_COEFFICIENT
 
 
 def _symmetric_pays(n: int, matrices: int) -> bool:
-    """Skipping the tiles below the diagonal only shortens a product that has more than one wave of 256 x 256
-    tiles to begin with (74 CTA pairs); below that the extra mirror launch costs more than it saves (measured:
-    2048 x 2048 slower, 4096 x 4096 1.35x faster than the full products)."""
-    return SYMMETRIC_PRODUCTS and matrices * (n // 256) ** 2 >= 148
+    """Skipping the tiles below the diagonal shortens a product that has more than one wave of 256 x 256 tiles
+    (74 CTA pairs); with fewer, the tiles above the diagonal take as long as all of them and are stored twice."""
+    return SYMMETRIC_PRODUCTS and matrices * (n / 256) ** 2 > 74
 
 
 def newton_schulz_sm100(x: torch.Tensor, coefficients=DEFAULT_NS_COEFFICIENTS, steps: int = 5) -> torch.Tensor:
