@@ -3,7 +3,7 @@
 // Input is the fused projection buffer qkv [T, 3H] (row = b*S + s; q heads, then k heads, then v heads,
 // RoPE already applied); output is [T, H] plus the per-row log-sum-exp the backward needs.
 //
-// Forward, one CTA per (batch, head, 128-query tile), 192 threads:
+// Forward for small grids, one CTA per (batch, head, 128-query tile), 320 threads (larger grids: attn_fwd2_kernel):
 //   warp 0   : TMA producer (Q once, then K/V tiles of 128 keys through a 2-stage ring)
 //   warp 1   : tcgen05.mma issuer.  S_j = Q K_j^T goes to one of two TMEM buffers so that S_{j+1} is
 //              computed while the softmax of tile j runs; O += P_j V_j accumulates in TMEM.
@@ -281,6 +281,248 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs p
         }
       }
       if (half == 0 && row_ok && p.lse) p.lse[((long long)b * p.nH + h) * p.S + qi] = (m_used + log2f(l)) * 0.6931471805599453f;
+    }
+  }
+  if (*abort_flag) __nanosleep(1000000);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// Forward for grids that fill the chip: one CTA per (batch, head, 256 queries), two 128-query tiles in flight.
+// One tile's softmax alone leaves the tensor pipe idle while it runs and waits while the pipe works; with two tiles
+// the products of one run beside the softmax of the other.  A thread owns a whole query row (no exchange between
+// threads, no block barrier in the loop) and P goes back to tensor memory over the scores it came from, so it
+// never touches shared memory.  Tensor memory: S0 | S1 | O0 | O1, 128 columns each; P_t packs into the first 64
+// columns of S_t.  Per 128 keys and 2 x 128 queries the tensor pipe needs 2048 cycles and the exponentials as many:
+// both bound it.  Measured (one tile per block -> two): 32 heads of 16384 rows 2476 -> 1791 us, 1228 TFLOP/s; 16 heads
+// of 2 x 4096 rows 212 -> 141 us; of 4 x 1024 47 -> 33 us; of 3 x 1333 56 -> 41 us.
+struct AttnFwd2Smem {
+  static constexpr int kQ = 0;                          // 2 query tiles
+  static constexpr int kK = kQ + 2 * kTileBytes;        // 2 stages
+  static constexpr int kV = kK + 2 * kTileBytes;        // 2 stages
+  static constexpr int kBars = kV + 2 * kTileBytes;
+  static constexpr int kBytes = kBars + 256 + 1024;
+};
+
+constexpr int kFwd2Threads = 384;     // warp 0 TMA, warp 1 MMA, 2 and 3 idle, warps 4-7 and 8-11 the two tiles' softmax
+// A row of 128 scores and their packed results need more than the 168 registers per thread of a 384-thread block,
+// so the first warpgroup hands registers to the other two: 128 * 48 + 256 * 224 = 63,488 of the launch's 64,512.
+constexpr int kFwd2RegsIssue = 48, kFwd2RegsSoftmax = 224;
+
+// D[128 x 128] (+)= P[128 x 128 (packed bf16 pairs in tensor memory)] * V[128 keys x 128 (N contiguous)]
+__device__ __forceinline__ void mma_pv_ts(uint32_t tmem_d, uint32_t tmem_p, uint32_t v_base, bool accumulate) {
+  constexpr uint32_t idesc = make_idesc_bf16(128, 128, false, true);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const uint64_t bd = make_smem_desc_sw128(v_base + k * 2048, kHalfTile, 1024);
+    umma_f16_ts(tmem_d, tmem_p + k * 8, bd, idesc, (accumulate || k > 0) ? 1u : 0u);
+  }
+}
+
+__global__ void __launch_bounds__(kFwd2Threads, 1)
+attn_fwd2_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs p, const int heads_per_group) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + AttnFwd2Smem::kBars);
+  uint64_t* q_full = bars;             // [1]
+  uint64_t* k_full = bars + 1;         // [2]
+  uint64_t* k_empty = bars + 3;        // [2]
+  uint64_t* v_full = bars + 5;         // [2]
+  uint64_t* v_empty = bars + 7;        // [2]
+  uint64_t* s_full = bars + 9;         // [2] per query tile
+  uint64_t* p_full = bars + 11;        // [2] per query tile, count 128
+  uint64_t* o_done = bars + 13;        // [2] per query tile: its last product has finished
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // Blocks are numbered so that, within a group of heads whose K and V fit the L2 together, the late (long) query
+  // tiles of all heads come first and the short ones fill the end of the grid.
+  const int nq = (p.S + 2 * kBq - 1) / (2 * kBq), nheads = p.nH * p.B;
+  const int grp = (int)blockIdx.x / (heads_per_group * nq);
+  const int in_grp = (int)blockIdx.x - grp * heads_per_group * nq;
+  const int gheads = min(heads_per_group, nheads - grp * heads_per_group);
+  const int qt = nq - 1 - in_grp / gheads;
+  const int bh = grp * heads_per_group + in_grp % gheads;
+  const int b = bh / p.nH, h = bh - b * p.nH;
+  const int H = p.nH * kHd;
+  const int q0 = qt * 2 * kBq;
+  const int row_base = b * p.S;
+  const int n0 = q0 / kBk + 1;                                 // key tiles of query tile 0
+  const int n1 = q0 + kBq < p.S ? n0 + 1 : 0;                  // ... and of tile 1, if it has any row
+  const int n_max = n1 > 0 ? n1 : n0;
+
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int i = 0; i < 15; ++i) mbar_init(smem_u32(&bars[i]), (i == 11 || i == 12) ? 128 : 1);
+    mbar_fence_init();
+    tma_prefetch_desc(&tma_qkv);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(tmem_slot), 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t sQ = smem_u32(smem + AttnFwd2Smem::kQ), sK = smem_u32(smem + AttnFwd2Smem::kK),
+                 sV = smem_u32(smem + AttnFwd2Smem::kV);
+
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kFwd2RegsIssue));
+    if (warp == 0 && lane == 0) {
+      mbar_arrive_expect_tx(smem_u32(q_full), n1 > 0 ? 2 * kTileBytes : kTileBytes);
+      tma_load_tile(sQ, &tma_qkv, smem_u32(q_full), h * kHd, row_base + q0);
+      if (n1 > 0) tma_load_tile(sQ + kTileBytes, &tma_qkv, smem_u32(q_full), h * kHd, row_base + q0 + kBq);
+      for (int j = 0; j < n_max; ++j) {
+        const uint32_t s = j & 1, ph = (j >> 1) & 1;
+        if (!mbar_wait(smem_u32(&k_empty[s]), ph ^ 1, p.status, abort_flag)) break;
+        mbar_arrive_expect_tx(smem_u32(&k_full[s]), kTileBytes);
+        tma_load_tile(sK + s * kTileBytes, &tma_qkv, smem_u32(&k_full[s]), H + h * kHd, row_base + j * kBk);
+        if (!mbar_wait(smem_u32(&v_empty[s]), ph ^ 1, p.status, abort_flag)) break;
+        mbar_arrive_expect_tx(smem_u32(&v_full[s]), kTileBytes);
+        tma_load_tile(sV + s * kTileBytes, &tma_qkv, smem_u32(&v_full[s]), 2 * H + h * kHd, row_base + j * kBk);
+      }
+    } else if (warp == 1 && lane == 0) {
+      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
+      bool ok = mbar_wait(smem_u32(q_full), 0, p.status, abort_flag) &&
+                mbar_wait(smem_u32(&k_full[0]), 0, p.status, abort_flag);
+      if (ok) {
+        tc_fence_after();
+        for (int t = 0; t < (n1 > 0 ? 2 : 1); ++t) {
+          mma_tile_128(tmem_base + t * 128, sQ + t * kTileBytes, false, sK, false, idesc_s, false);
+          umma_commit(smem_u32(&s_full[t]));
+        }
+        umma_commit(smem_u32(&k_empty[0]));
+      }
+      for (int j = 0; j < n_max && ok; ++j) {
+        const uint32_t s = j & 1, ph = (j >> 1) & 1, s1 = (j + 1) & 1, ph1 = ((j + 1) >> 1) & 1;
+        if (!mbar_wait(smem_u32(&v_full[s]), ph, p.status, abort_flag)) { ok = false; break; }
+        if (j + 1 < n_max && !mbar_wait(smem_u32(&k_full[s1]), ph1, p.status, abort_flag)) { ok = false; break; }
+        for (int t = 0; t < 2; ++t) {
+          const int n = t == 0 ? n0 : n1;
+          if (j >= n) continue;
+          if (!mbar_wait(smem_u32(&p_full[t]), j & 1, p.status, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          // S_t's scores have all been read and P_t lies over them; the next scores may overwrite both because the
+          // tensor pipe runs a thread's products in the order they were issued
+          mma_pv_ts(tmem_base + 256 + t * 128, tmem_base + t * 128, sV + s * kTileBytes, j > 0);
+          if (j + 1 < n) {
+            mma_tile_128(tmem_base + t * 128, sQ + t * kTileBytes, false, sK + s1 * kTileBytes, false, idesc_s, false);
+            umma_commit(smem_u32(&s_full[t]));
+          } else {
+            umma_commit(smem_u32(&o_done[t]));
+          }
+        }
+        umma_commit(smem_u32(&v_empty[s]));
+        if (j + 1 < n_max) umma_commit(smem_u32(&k_empty[s1]));
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ softmax / epilogue: 4 warps per query tile
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFwd2RegsSoftmax));
+    const int t = (warp - 4) >> 2;
+    const int q = warp & 3;                      // TMEM lane quadrant this warp may access
+    const int r = q * 32 + lane;                 // query row inside the tile == TMEM lane
+    const int n = t == 0 ? n0 : n1;
+    const uint32_t tmem_s = tmem_base + t * 128 + ((uint32_t)(q * 32) << 16);
+    const uint32_t tmem_o = tmem_s + 256;
+    const int qi = q0 + t * kBq + r;
+    float m_used = -INFINITY, l = 0.f;
+    bool ok = true;
+    for (int j = 0; j < n; ++j) {
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[t]), j & 1, p.status, abort_flag))) { ok = false; break; }
+      tc_fence_after();
+      uint32_t u[128];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(tmem_s + c * 32, *reinterpret_cast<uint32_t(*)[32]>(u + c * 32));
+      tmem_ld_wait();
+      if (j == n - 1) {
+        const int kv0 = j * kBk;
+#pragma unroll
+        for (int e = 0; e < 128; ++e)
+          if (kv0 + e > qi) u[e] = 0xff800000u;
+      }
+      float m4[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) m4[e] = fmaxf(__uint_as_float(u[e]), __uint_as_float(u[4 + e]));
+#pragma unroll
+      for (int e = 8; e < 128; e += 8)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          m4[k] = fmaxf(fmaxf(m4[k], __uint_as_float(u[e + k])), __uint_as_float(u[e + 4 + k]));
+      float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
+      if (mx == -INFINITY) mx = 0.f;
+      const float m_new = fmaxf(m_used, mx);
+      const bool need = (j > 0) && (m_new - m_used > 8.f);
+      const bool any_need = __any_sync(0xffffffffu, need);
+      const float m_next = (j == 0 || any_need) ? m_new : m_used;
+      const float factor = (j == 0) ? 0.f : exp2f(m_used - m_next);
+      m_used = m_next;
+      const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2), nm2 = pack_f32x2(-m_next, -m_next);
+      uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t pk[32];
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+          float x0, x1;
+          unpack_f32x2(fma_f32x2(pack_u32x2(u[half * 64 + 2 * e], u[half * 64 + 2 * e + 1]), sc2, nm2), x0, x1);
+          x0 = exp2f(x0);
+          x1 = exp2f(x1);
+          sum2[e & 3] = add_f32x2(sum2[e & 3], pack_f32x2(x0, x1));
+          pk[e] = pack_bf16x2(x0, x1);
+        }
+        tmem_st_32x32b_x32(tmem_s + half * 32, pk);
+      }
+      float a0, a1;
+      unpack_f32x2(add_f32x2(add_f32x2(sum2[0], sum2[1]), add_f32x2(sum2[2], sum2[3])), a0, a1);
+      l = l * factor + (a0 + a1);
+      if (any_need) {
+        // the scores just read were computed after the previous P V product, so O is complete
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t o[32];
+          tmem_ld_32x32b_x32(tmem_o + c * 32, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * factor);
+          tmem_st_32x32b_x32(tmem_o + c * 32, o);
+        }
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(smem_u32(&p_full[t]));
+    }
+    if (ok && n > 0) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&o_done[t]), 0, p.status, abort_flag));
+    if (ok && n > 0) {
+      tc_fence_after();
+      const float inv = 1.f / l;
+      const bool row_ok = qi < p.S;
+      __nv_bfloat16* orow = p.out + (long long)(row_base + qi) * p.ld_out + h * kHd;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t o[32];
+        tmem_ld_32x32b_x32(tmem_o + c * 32, o);
+        tmem_ld_wait();
+        if (row_ok) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            uint4 w;
+            w.x = pack_bf16x2(__uint_as_float(o[g * 8 + 0]) * inv, __uint_as_float(o[g * 8 + 1]) * inv);
+            w.y = pack_bf16x2(__uint_as_float(o[g * 8 + 2]) * inv, __uint_as_float(o[g * 8 + 3]) * inv);
+            w.z = pack_bf16x2(__uint_as_float(o[g * 8 + 4]) * inv, __uint_as_float(o[g * 8 + 5]) * inv);
+            w.w = pack_bf16x2(__uint_as_float(o[g * 8 + 6]) * inv, __uint_as_float(o[g * 8 + 7]) * inv);
+            *reinterpret_cast<uint4*>(orow + c * 32 + g * 8) = w;
+          }
+        }
+      }
+      if (row_ok && p.lse) p.lse[((long long)b * p.nH + h) * p.S + qi] = (m_used + log2f(l)) * 0.6931471805599453f;
     }
   }
   if (*abort_flag) __nanosleep(1000000);
@@ -644,6 +886,15 @@ __global__ void attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ dout, lon
 
 using namespace mfsdp;
 
+// Bytes of K and V that a group of heads may occupy (half of the 126 MB L2, the rest is for Q, O and the other die).
+constexpr long long kKvInL2 = 64LL << 20;
+
+// A grid of at most one 128-query tile per SM is as long as its longest tile, which two threads per row finish sooner
+// (16 heads of 1024 rows: 20 us in one-tile blocks, 25 in two); above that two tiles per block win at every size tried.
+static bool attn_fwd_two_tiles(int B, int S, int nH) {
+  return (long long)((S + kBq - 1) / kBq) * nH * B > 148;
+}
+
 // qkv: [B*S, 3*nH*128] bf16 (row stride ld_qkv elements); out: [B*S, nH*128]; lse: [B, nH, S] fp32.
 MFSDP_API int mfsdp_attention_fwd(const void* qkv, void* out, float* lse, int B, int S, int nH, long long ld_qkv,
                                   long long ld_out, float softmax_scale, int* status, cudaStream_t st) {
@@ -655,6 +906,8 @@ MFSDP_API int mfsdp_attention_fwd(const void* qkv, void* out, float* lse, int B,
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnFwdSmem::kBytes);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(attn_fwd2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnFwd2Smem::kBytes);
     if (e != cudaSuccess) return (int)e;
     attr = true;
   }
@@ -662,6 +915,14 @@ MFSDP_API int mfsdp_attention_fwd(const void* qkv, void* out, float* lse, int B,
   a.B = B; a.S = S; a.nH = nH;
   a.scale_log2 = softmax_scale * kLog2e;
   a.out = (__nv_bfloat16*)out; a.ld_out = ld_out; a.lse = lse; a.status = status;
+  if (attn_fwd_two_tiles(B, S, nH)) {
+    const int nq = (S + 2 * kBq - 1) / (2 * kBq);
+    long long group = kKvInL2 / ((long long)S * kHd * 2 * 2);
+    if (group < 1) group = 1;
+    if (group > (long long)B * nH) group = (long long)B * nH;
+    attn_fwd2_kernel<<<(unsigned)(nq * B * nH), kFwd2Threads, AttnFwd2Smem::kBytes, st>>>(map, a, (int)group);
+    return (int)cudaGetLastError();
+  }
   dim3 grid((S + kBq - 1) / kBq, nH, B);
   attn_fwd_kernel<<<grid, kAttnThreads, AttnFwdSmem::kBytes, st>>>(map, a);
   return (int)cudaGetLastError();

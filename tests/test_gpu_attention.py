@@ -76,3 +76,44 @@ def test_attention_bwd_matches_fp32(B, S, nH):
     assert err < 6e-2 * max(1.0, ref_g.abs().max().item() / 4), err
     rel = (dqkv.float() - ref_g).norm() / ref_g.norm()
     assert rel.item() < 2e-2, rel.item()
+
+
+@pytest.mark.parametrize("B,S,nH,heads", [(1, 1, 150, (0, 149)), (2, 100, 80, (3, 79)), (1, 128, 150, (0, 7)), (1, 129, 80, (0, 79)),
+                                          (2, 255, 40, (1, 39)), (1, 257, 50, (0, 49)), (1, 385, 40, (2, 39)),
+                                          (3, 1333, 16, (0, 15)), (1, 8192, 20, (0, 15, 16, 19))])
+def test_attention_fwd_two_tiles_per_block(B, S, nH, heads):
+    """Grids of more than 148 query tiles take the kernel with two of them per block: a lone tile, a second tile of one
+    row, odd and even tile counts, and a last group of heads that is not full.  Bounds as for the other kernel."""
+    from matrix_fsdp_b200.ops import attention as A
+    from matrix_fsdp_b200.ops import kernels as K
+
+    assert (S + 127) // 128 * B * nH > 148
+    torch.manual_seed(0)
+    hd = 128
+    qkv = torch.randn(B * S, 3 * nH * hd, device="cuda", dtype=torch.bfloat16)
+    out, lse = A.attention_fwd(qkv, B, S, nH, hd)
+    K.check_status()
+    assert torch.isfinite(out).all() and torch.isfinite(lse).all()
+    for b in range(B):
+        for h in heads:
+            one = torch.cat([qkv[b * S:(b + 1) * S, (i * nH + h) * hd:(i * nH + h + 1) * hd] for i in range(3)], dim=1)
+            ref_o, ref_lse = _ref(one, 1, S, 1, hd)
+            assert (out[b * S:(b + 1) * S, h * hd:(h + 1) * hd].float() - ref_o).abs().max().item() < 3e-2
+            assert (lse[b, h] - ref_lse[0, 0]).abs().max().item() < 2e-3
+
+
+def test_attention_fwd_two_tiles_rescale():
+    """Scores that grow along the key axis, in steps that force the rescaling of O in some warps and not in others."""
+    from matrix_fsdp_b200.ops import attention as A
+    from matrix_fsdp_b200.ops import kernels as K
+
+    torch.manual_seed(1)
+    B, S, nH, hd = 1, 700, 32, 128
+    qkv = torch.randn(B * S, 3 * nH * hd, device="cuda", dtype=torch.bfloat16)
+    ramp = torch.linspace(0.2, 6.0, S, device="cuda")[:, None]
+    qkv[:, nH * hd:2 * nH * hd] = (qkv[:, nH * hd:2 * nH * hd].float() * ramp).bfloat16()
+    out, lse = A.attention_fwd(qkv, B, S, nH, hd)
+    K.check_status()
+    ref_o, ref_lse = _ref(qkv, B, S, nH, hd)
+    assert (out.float() - ref_o).abs().max().item() < 4e-2
+    assert (lse - ref_lse).abs().max().item() < 5e-3
