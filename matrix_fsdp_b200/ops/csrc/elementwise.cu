@@ -703,6 +703,21 @@ __global__ void cast_f32_bf16_kernel(const float* __restrict__ src, __nv_bfloat1
   }
 }
 
+// bf16 -> fp32, 8 elements per access (reduced gradients into the fp32 shard that the optimizer reads).  Bound by
+// memory; the library's converting copy moved 60 M elements in 179 us, 2.0 TB/s.
+__global__ void __launch_bounds__(256) cast_bf16_f32_kernel(const __nv_bfloat16* __restrict__ src, float* __restrict__ dst, long long n) {
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long nv = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0 ? n >> 3 : 0;
+#pragma unroll 4
+  for (long long i = tid; i < nv; i += stride) {
+    float f[8];
+    load8(src + i * 8, f);
+    store8(dst + i * 8, f);
+  }
+  for (long long i = nv * 8 + tid; i < n; i += stride) dst[i] = __bfloat162float(src[i]);
+}
+
 static inline int grid_for(long long work, int threads, int max_blocks = 148 * 8) {
   long long b = (work + threads - 1) / threads;
   if (b < 1) b = 1;
@@ -1059,6 +1074,12 @@ MFSDP_API int mfsdp_copy_segments(const void* src, void* dst, const long long* s
 MFSDP_API int mfsdp_cast_f32_bf16(const float* src, void* dst, long long n, cudaStream_t st) {
   if (n <= 0) return 0;
   cast_f32_bf16_kernel<<<grid_for(n / 4 + 1, 256, 148 * 8), 256, 0, st>>>(src, (__nv_bfloat16*)dst, n);
+  return (int)cudaGetLastError();
+}
+
+MFSDP_API int mfsdp_cast_bf16_f32(const void* src, float* dst, long long n, cudaStream_t st) {
+  if (n <= 0) return 0;
+  cast_bf16_f32_kernel<<<grid_for(n / 8 + 1, 256, 148 * 8), 256, 0, st>>>((const __nv_bfloat16*)src, dst, n);
   return (int)cudaGetLastError();
 }
 

@@ -407,3 +407,9 @@ def cast_f32_bf16(src: torch.Tensor, dst: torch.Tensor) -> None:
     assert src.dtype == torch.float32 and dst.dtype == torch.bfloat16 and src.numel() == dst.numel()
     _lib.check(_L().mfsdp_cast_f32_bf16(src.data_ptr(), dst.data_ptr(), src.numel(), _stream()),
                "cast_f32_bf16")
+
+
+def cast_bf16_f32(src: torch.Tensor, dst: torch.Tensor) -> None:
+    assert src.dtype == torch.bfloat16 and dst.dtype == torch.float32 and src.numel() == dst.numel()
+    assert src.is_contiguous() and dst.is_contiguous()
+    _lib.check(_L().mfsdp_cast_bf16_f32(src.data_ptr(), dst.data_ptr(), src.numel(), _stream()), "cast_bf16_f32")

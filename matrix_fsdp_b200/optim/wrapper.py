@@ -387,9 +387,10 @@ class MixedMuonAdamWOptimizer:
             self.adamw.step()
             lp_of = getattr(self.adamw, "_low_precision_of", None)
             if lp_of is not None:
+                written = getattr(self.adamw, "lp_written", ())
                 for g in self.adamw.param_groups:
                     for p in g["params"]:
-                        if p.grad is not None and p.numel():
+                        if p.grad is not None and p.numel() and id(p) not in written:
                             lp = lp_of(p)
                             if lp is not None:
                                 lp.copy_(p.data)

@@ -172,10 +172,21 @@ def scatter_local_segments(shard: torch.Tensor, full: torch.Tensor, segments: Se
         full[s.global_start:s.global_end].copy_(shard[s.local_start:s.local_end])
 
 
+def _copy_segment(dst: torch.Tensor, src: torch.Tensor) -> None:
+    if src.is_cuda and dst.device == src.device and src.dtype == torch.bfloat16 and dst.dtype == torch.float32 \
+            and src.is_contiguous() and dst.is_contiguous():
+        from ..ops import kernels, lib
+
+        if lib.available() and not lib.disabled_by_env():
+            kernels.cast_bf16_f32(src, dst)
+            return
+    dst.copy_(src)
+
+
 def gather_local_segments(full: torch.Tensor, shard: torch.Tensor, segments: Sequence[LayoutSegment]) -> None:
     """``shard[l0:l1] = full[g0:g1]`` for every segment."""
     for s in segments:
-        shard[s.local_start:s.local_end].copy_(full[s.global_start:s.global_end])
+        _copy_segment(shard[s.local_start:s.local_end], full[s.global_start:s.global_end])
 
 
 # --------------------------------------------------------------------------- all-gather

@@ -403,3 +403,37 @@ def test_grouped_gemms_on_cta_pairs(K):
     K.check_status()
     ref3 = torch.bmm(a2.view(G, kk, M2).float().transpose(1, 2), b2.view(G, kk, N2).float())
     assert _rel_err(o3, ref3) < 1e-2
+
+
+@pytest.mark.parametrize("n,shift", [(1, 0), (7, 0), (8, 0), (4099, 0), (4096, 1), (4096, 4), (1 << 20, 0)])
+def test_cast_bf16_f32(K, n, shift):
+    """Every bf16 value has the same fp32 value: exact, with and without 16-byte aligned bases."""
+    src = torch.randn(n + shift, device="cuda").bfloat16()[shift:]
+    dst = torch.empty(n + shift, device="cuda")[shift:]
+    K.cast_bf16_f32(src, dst)
+    assert torch.equal(dst, src.float())
+
+
+@pytest.mark.parametrize("n,with_lp,aligned", [(5, True, True), (1024, True, True), (1001, False, True), (1000, True, False)])
+def test_adamw_of_parameters_outside_units(n, with_lp, aligned):
+    """One fused launch per parameter against the torch-op update (fp32, terms of one sum in another order: 1e-6),
+    whose path unaligned views keep."""
+    from matrix_fsdp_b200.optim.flat import FlatShardedAdamW, _adamw_reference_
+
+    torch.manual_seed(0)
+    base = torch.randn(n + 1, device="cuda")
+    p = torch.nn.Parameter(base[0 if aligned else 1:][:n])
+    lp = torch.zeros(n, device="cuda", dtype=torch.bfloat16)
+    opt = FlatShardedAdamW([p], lr=1e-2, betas=(0.9, 0.95), weight_decay=0.1)
+    if with_lp:
+        opt._low_precision_of = lambda _: lp
+    want, m, v = p.detach().clone(), torch.zeros_like(p.data), torch.zeros_like(p.data)
+    for step in (1, 2):
+        p.grad = torch.randn(n, device="cuda")
+        _adamw_reference_(want, m, v, p.grad, lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=step,
+                          grad_scale=1.0)
+        opt.step()
+        assert (p.detach() - want).abs().max() <= 1e-6 * want.abs().max()
+        assert (id(p) in opt.lp_written) == (with_lp and aligned)
+        if with_lp and aligned:
+            assert torch.equal(lp, p.detach().bfloat16())
