@@ -94,8 +94,10 @@ def attention_bwd(dout: torch.Tensor, qkv: torch.Tensor, out: torch.Tensor, lse:
     scale = 1.0 / math.sqrt(head_dim) if softmax_scale is None else float(softmax_scale)
     dout = dout.contiguous()
     out = out if out.stride(0) == dout.stride(0) else out.contiguous()
+    if out.data_ptr() % 16:                      # the kernels read 16-byte vectors of it
+        out = out.clone()
     dqkv = torch.empty_like(qkv, memory_format=torch.contiguous_format)
-    scratch = torch.empty(2 * batch * n_heads * seq, dtype=torch.float32, device=qkv.device)
+    scratch = torch.empty(2 * batch * n_heads * ((seq + 127) // 128 * 128), dtype=torch.float32, device=qkv.device)
     status = K.status_word(qkv.device)
     lib = _lib.load()
     _lib.check(lib.mfsdp_attention_bwd(dout.data_ptr(), qkv.data_ptr(), out.data_ptr(), lse.data_ptr(),

@@ -310,8 +310,8 @@ struct AttnFwd2Smem {
 
 constexpr int kFwd2Threads = 384;     // warp 0 TMA, warp 1 MMA, 2 and 3 idle, warps 4-7 and 8-11 the two tiles' softmax
 // A row of 128 scores and their packed results need more than the 168 registers per thread of a 384-thread block,
-// so the first warpgroup hands registers to the other two: 128 * 48 + 256 * 224 = 63,488 of the launch's 64,512.
-constexpr int kFwd2RegsIssue = 48, kFwd2RegsSoftmax = 224;
+// so the first warpgroup hands registers to the other two: 128 * 56 + 256 * 224 = the launch's 64,512.
+constexpr int kRegsIssue = 56, kRegsSoftmax = 224;
 
 // D[128 x 128] (+)= P[128 x 128 (packed bf16 pairs in tensor memory)] * V[128 keys x 128 (N contiguous)]
 __device__ __forceinline__ void mma_pv_ts(uint32_t tmem_d, uint32_t tmem_p, uint32_t v_base, bool accumulate) {
@@ -374,7 +374,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs 
                  sV = smem_u32(smem + AttnFwd2Smem::kV);
 
   if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kFwd2RegsIssue));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
     if (warp == 0 && lane == 0) {
       mbar_arrive_expect_tx(smem_u32(q_full), n1 > 0 ? 2 * kTileBytes : kTileBytes);
       tma_load_tile(sQ, &tma_qkv, smem_u32(q_full), h * kHd, row_base + q0);
@@ -425,7 +425,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs 
     }
   } else {
     // ------------------------------------------------------------ softmax / epilogue: 4 warps per query tile
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFwd2RegsSoftmax));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
     const int t = (warp - 4) >> 2;
     const int q = warp & 3;                      // TMEM lane quadrant this warp may access
     const int r = q * 32 + lane;                 // query row inside the tile == TMEM lane
@@ -536,121 +536,92 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs 
 
 
 // =============================================================================== backward
-// Two kernels without atomics, sharing one body:
-//   DQ = false: one CTA per (batch, head, 128-key tile).  K_j and V_j stay in shared memory; the
-//               query axis streams in tiles of 64 rows (Q_t, dO_t).  S^T = K_j Q_t^T and
-//               dP^T = V_j dO_t^T land in TMEM (thread = key row), P^T and dS^T go to swizzled shared
-//               tiles, dV += P^T dO_t and dK += dS^T Q_t accumulate in TMEM.
-//   DQ = true : one CTA per (batch, head, 128-query tile).  Q_i and dO_i stay; keys stream in tiles
-//               of 64 (K_t, V_t).  S = Q_i K_t^T, dP = dO_i V_t^T, dS to shared, dQ += dS K_t.
-// The 64-wide streamed tiles leave room for two TMEM buffers of S/dP (2 x 128 columns) beside the
-// two 128-column accumulators, and for two stages of every streamed shared tile, so the tensor pipe
-// works on tile t+1 while the softmax threads turn tile t into P / dS.
-constexpr int kBt = 64;                       // streamed rows per iteration
-constexpr int kStreamBytes = kBt * 128 * 2;   // one streamed [64 x 128] tile = two 8 KB chunks
-constexpr int kPBytes = 128 * kBt * 2;        // one [128 x 64] P or dS tile (single 64-column chunk)
+// Two kernels without atomics (the sums have one order in every run), sharing one body:
+//   DQ = false: one CTA per (batch, head, 128-key tile).  K_j and V_j stay in shared memory, the query axis streams
+//               in tiles of 128 rows (Q_i, dO_i).  S^T = K_j Q_i^T and dP^T = V_j dO_i^T land in TMEM (thread = key
+//               row, two threads per row), P^T and dS^T go back over them as bf16, dV += P^T dO_i and dK += dS^T Q_i
+//               accumulate in TMEM.
+//   DQ = true : one CTA per (batch, head, 128-query tile).  Q_i and dO_i stay, keys stream (K_j, V_j).
+//               S = Q_i K_j^T, dP = dO_i V_j^T, dQ += dS K_j.
+// Bound by the tensor pipe (four and three 128 x 128 x 128 products per tile, 512 cycles each).  Its queue never runs
+// dry although every buffer is single: while the threads turn dP into dS the pipe adds to dV and computes the next S,
+// and while they take exponentials of that S it adds to dK / dQ and computes the next dP.  128-wide streamed tiles,
+// because a 64-wide second operand makes the products wait for shared memory (A and B together 192 B per cycle).
+// The row statistics of a streamed tile arrive with it, in the same barrier, so no thread waits for another.
+constexpr int kBwdThreads = 384;      // warp 0 TMA, warp 1 MMA, 2 and 3 idle, warps 4-11 P and dS
+constexpr int kStatBytes = 128 * 4;   // one row statistic of a streamed tile
 
 struct AttnBwdArgs {
   int B, S, nH;
+  long long Sp;              // row pitch of the statistics: S rounded up to 128
   float scale, scale_log2;
-  const float* lse2;         // [B, nH, S] log-sum-exp in log2 units
-  const float* delta;        // [B, nH, S] rowsum(dO * O)
+  const float* nlse2;        // [B * nH, Sp] minus log-sum-exp in log2 units
+  const float* ndelta;       // [B * nH, Sp] minus rowsum(dO * O)
   __nv_bfloat16* dqkv;       // [T, 3H]
   long long ld_dqkv;
   int* status;
+  int heads_per_group;
 };
-
-constexpr int kBwdStages = 3;   // streamed-tile ring: deep enough to hide the TMA latency behind two tiles of work
 
 struct AttnBwdSmem {
   static constexpr int kA0 = 0;
   static constexpr int kA1 = kA0 + kTileBytes;
-  static constexpr int kB = kA1 + kTileBytes;             // kBwdStages stages x (B0, B1)
-  static constexpr int kP = kB + kBwdStages * 2 * kStreamBytes;   // 2 stages x (P, dS)
-  static constexpr int kRow = kP + 4 * kPBytes;           // 2 stages x 128 floats (lse2 | delta of the streamed rows)
-  static constexpr int kBars = kRow + 2 * 128 * 4;
+  static constexpr int kB = kA1 + kTileBytes;             // 2 stages x (B0, B1)
+  static constexpr int kRow = kB + 4 * kTileBytes;        // 2 stages x (nlse2, ndelta)
+  static constexpr int kBars = kRow + 4 * kStatBytes;
   static constexpr int kBytes = kBars + 256 + 1024;
 };
 
-// [128 x 128] stationary tile through a [64 rows x 64 cols] box map: four boxes.
-__device__ __forceinline__ void tma_load_tile_4(uint32_t dst, const CUtensorMap* map, uint32_t bar, int col0, int row0) {
-  tma_load_2d(dst, map, bar, col0, row0);
-  tma_load_2d(dst + 8192, map, bar, col0, row0 + 64);
-  tma_load_2d(dst + kHalfTile, map, bar, col0 + 64, row0);
-  tma_load_2d(dst + kHalfTile + 8192, map, bar, col0 + 64, row0 + 64);
-}
-// [64 x 128] streamed tile: two boxes.
-__device__ __forceinline__ void tma_load_stream(uint32_t dst, const CUtensorMap* map, uint32_t bar, int col0, int row0) {
-  tma_load_2d(dst, map, bar, col0, row0);
-  tma_load_2d(dst + 8192, map, bar, col0 + 64, row0);
-}
-
-// D[128 x 64] = A[128 x 128 (K-major)] * B[64 x 128 (K-major)]^T
-__device__ __forceinline__ void mma_sdp(uint32_t tmem_d, uint32_t a_base, uint32_t b_base) {
-  constexpr uint32_t idesc = make_idesc_bf16(128, kBt, false, false);
+// D[128 x 128] (+)= P[128 x 128] * B[128 rows along K x 128, N contiguous].  The two threads of a row have each packed
+// their 64 elements into the first 32 columns of their own half.
+__device__ __forceinline__ void mma_acc_ts(uint32_t tmem_d, uint32_t tmem_p, uint32_t b_base, bool accumulate) {
+  constexpr uint32_t idesc = make_idesc_bf16(128, 128, false, true);
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    const uint64_t ad = make_smem_desc_sw128(a_base + (k >> 2) * kHalfTile + (k & 3) * 32, 16, 1024);
-    const uint64_t bd = make_smem_desc_sw128(b_base + (k >> 2) * 8192 + (k & 3) * 32, 16, 1024);
-    umma_f16_ss(tmem_d, ad, bd, idesc, k > 0 ? 1u : 0u);
-  }
-}
-// Same product with the A operand (P or dS as packed bf16 pairs) read from tensor memory: the thread that
-// owns row r stored elements [32h, 32h+32) of its row as 16 packed columns at column offset 32h, so
-// k-step kk (16 elements) starts at column (kk >> 1) * 32 + (kk & 1) * 8.
-__device__ __forceinline__ void mma_acc_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_base, bool accumulate) {
-  constexpr uint32_t idesc = make_idesc_bf16(128, 128, false, true);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const uint64_t bd = make_smem_desc_sw128(b_base + k * 2048, 8192, 1024);
-    umma_f16_ts(tmem_d, tmem_a + (k >> 1) * 32 + (k & 1) * 8, bd, idesc, (accumulate || k > 0) ? 1u : 0u);
-  }
-}
-// D[128 x 128] (+)= P[128 x 64 (K-major)] * B[64 x 128 (rows along K, N contiguous)]
-__device__ __forceinline__ void mma_acc(uint32_t tmem_d, uint32_t p_base, uint32_t b_base, bool accumulate) {
-  constexpr uint32_t idesc = make_idesc_bf16(128, 128, false, true);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const uint64_t ad = make_smem_desc_sw128(p_base + k * 32, 16, 1024);
-    const uint64_t bd = make_smem_desc_sw128(b_base + k * 2048, 8192, 1024);
-    umma_f16_ss(tmem_d, ad, bd, idesc, (accumulate || k > 0) ? 1u : 0u);
+    const uint64_t bd = make_smem_desc_sw128(b_base + k * 2048, kHalfTile, 1024);
+    umma_f16_ts(tmem_d, tmem_p + (k >> 2) * 64 + (k & 3) * 8, bd, idesc, (accumulate || k > 0) ? 1u : 0u);
   }
 }
 
-// PT: P and dS stay in tensor memory (written over the S / dP columns their thread just read) and feed
-// the accumulation MMAs from there; otherwise they go through swizzled shared tiles.
-template <bool DQ, bool PT>
-__global__ void __launch_bounds__(kAttnThreads, 1)
+template <bool DQ>
+__global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_constant__ CUtensorMap tma_do,
                 const AttnBwdArgs p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + AttnBwdSmem::kBars);
   uint64_t* stat_full = bars;          // [1]
-  uint64_t* b_full = bars + 1;         // [3]
-  uint64_t* b_empty = bars + 4;        // [3] streamed tiles of a stage consumed by both of their MMAs
-  uint64_t* sdp_full = bars + 7;       // [2]
-  uint64_t* p_full = bars + 9;         // [2] count 256
-  uint64_t* p_free = bars + 11;        // [2] P / dS tiles of a stage consumed
-  uint64_t* acc_done = bars + 13;      // [1]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* b_full = bars + 1;         // [2]
+  uint64_t* b_empty = bars + 3;        // [2] all products of a streamed tile have finished
+  uint64_t* s_full = bars + 5;         // [1]
+  uint64_t* dp_full = bars + 6;        // [1]
+  uint64_t* p_ready = bars + 7;        // [1] count 256: S read, P written
+  uint64_t* ds_ready = bars + 8;       // [1] count 256: dP read, dS written
+  uint64_t* acc_done = bars + 9;       // [1]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* row_vals = reinterpret_cast<float*>(smem + AttnBwdSmem::kRow);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y, b = blockIdx.z;
+  // Blocks in the order of attn_fwd2_kernel: per group of heads the long tiles first.
+  const int nt = (p.S + 127) / 128, nheads = p.nH * p.B;
+  const int grp = (int)blockIdx.x / (p.heads_per_group * nt);
+  const int in_grp = (int)blockIdx.x - grp * p.heads_per_group * nt;
+  const int gheads = min(p.heads_per_group, nheads - grp * p.heads_per_group);
+  const int nth = in_grp / gheads;
+  const int bh = grp * p.heads_per_group + in_grp % gheads;
+  const int b = bh / p.nH, h = bh - b * p.nH;
   const int H = p.nH * kHd;
   const int row_base = b * p.S;
-  // DQ: stationary tile = queries [r0, r0+128), streamed = keys.  Otherwise stationary = keys.
-  const int tile = DQ ? ((int)gridDim.x - 1 - (int)blockIdx.x) : (int)blockIdx.x;
+  // DQ: stationary tile = queries [r0, r0 + 128), streamed = keys up to the diagonal; otherwise stationary = keys,
+  // streamed = queries from the diagonal on.
+  const int tile = DQ ? nt - 1 - nth : nth;
   const int r0 = tile * 128;
-  const int t_begin = DQ ? 0 : (r0 / kBt);
-  const int t_end = DQ ? ((min(r0 + 128, p.S) + kBt - 1) / kBt) : ((p.S + kBt - 1) / kBt);
-  const int T = t_end - t_begin;
+  const int t_begin = DQ ? 0 : tile;
+  const int T = DQ ? tile + 1 : nt - tile;
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    for (int i = 0; i < 14; ++i) mbar_init(smem_u32(&bars[i]), (i == 9 || i == 10) ? 256 : 1);
+    for (int i = 0; i < 10; ++i) mbar_init(smem_u32(&bars[i]), (i == 7 || i == 8) ? 256 : 1);
     mbar_fence_init();
     tma_prefetch_desc(&tma_qkv);
     tma_prefetch_desc(&tma_do);
@@ -663,164 +634,147 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_acc0 = tmem_base + 256, tmem_acc1 = tmem_base + 384;
+  const uint32_t tmem_dp = tmem_base + 128, tmem_acc0 = tmem_base + 256, tmem_acc1 = tmem_base + 384;
   const uint32_t sA0 = smem_u32(smem + AttnBwdSmem::kA0), sA1 = smem_u32(smem + AttnBwdSmem::kA1),
-                 sB = smem_u32(smem + AttnBwdSmem::kB), sP = smem_u32(smem + AttnBwdSmem::kP);
+                 sB = smem_u32(smem + AttnBwdSmem::kB), sRow = smem_u32(smem + AttnBwdSmem::kRow);
 
-  if (warp == 0) {
-    if (lane == 0) {
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
+    if (warp == 0 && lane == 0) {
       mbar_arrive_expect_tx(smem_u32(stat_full), 2 * kTileBytes);
       if (DQ) {
-        tma_load_tile_4(sA0, &tma_qkv, smem_u32(stat_full), h * kHd, row_base + r0);          // Q_i
-        tma_load_tile_4(sA1, &tma_do, smem_u32(stat_full), h * kHd, row_base + r0);           // dO_i
+        tma_load_tile(sA0, &tma_qkv, smem_u32(stat_full), h * kHd, row_base + r0);          // Q_i
+        tma_load_tile(sA1, &tma_do, smem_u32(stat_full), h * kHd, row_base + r0);           // dO_i
       } else {
-        tma_load_tile_4(sA0, &tma_qkv, smem_u32(stat_full), H + h * kHd, row_base + r0);      // K_j
-        tma_load_tile_4(sA1, &tma_qkv, smem_u32(stat_full), 2 * H + h * kHd, row_base + r0);  // V_j
+        tma_load_tile(sA0, &tma_qkv, smem_u32(stat_full), H + h * kHd, row_base + r0);      // K_j
+        tma_load_tile(sA1, &tma_qkv, smem_u32(stat_full), 2 * H + h * kHd, row_base + r0);  // V_j
       }
       for (int i = 0; i < T; ++i) {
-        const uint32_t s = i % kBwdStages, ph = (i / kBwdStages) & 1;
+        const uint32_t s = i & 1, ph = (i >> 1) & 1;
         if (!mbar_wait(smem_u32(&b_empty[s]), ph ^ 1, p.status, abort_flag)) break;
-        mbar_arrive_expect_tx(smem_u32(&b_full[s]), 2 * kStreamBytes);
-        const int row = row_base + (t_begin + i) * kBt;
-        const uint32_t dst = sB + s * 2 * kStreamBytes;
+        const uint32_t bar = smem_u32(&b_full[s]), dst = sB + s * 2 * kTileBytes;
+        mbar_arrive_expect_tx(bar, 2 * kTileBytes + (DQ ? 0 : 2 * kStatBytes));
+        const int t0 = (t_begin + i) * 128, row = row_base + t0;
         if (DQ) {
-          tma_load_stream(dst, &tma_qkv, smem_u32(&b_full[s]), H + h * kHd, row);                     // K_t
-          tma_load_stream(dst + kStreamBytes, &tma_qkv, smem_u32(&b_full[s]), 2 * H + h * kHd, row);  // V_t
+          tma_load_tile(dst, &tma_qkv, bar, H + h * kHd, row);                       // K_t
+          tma_load_tile(dst + kTileBytes, &tma_qkv, bar, 2 * H + h * kHd, row);      // V_t
         } else {
-          tma_load_stream(dst, &tma_qkv, smem_u32(&b_full[s]), h * kHd, row);                         // Q_t
-          tma_load_stream(dst + kStreamBytes, &tma_do, smem_u32(&b_full[s]), h * kHd, row);           // dO_t
+          tma_load_tile(dst, &tma_qkv, bar, h * kHd, row);                           // Q_t
+          tma_load_tile(dst + kTileBytes, &tma_do, bar, h * kHd, row);               // dO_t
+          bulk_load(sRow + s * 2 * kStatBytes, p.nlse2 + (long long)bh * p.Sp + t0, kStatBytes, bar);
+          bulk_load(sRow + s * 2 * kStatBytes + kStatBytes, p.ndelta + (long long)bh * p.Sp + t0, kStatBytes, bar);
         }
       }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
+    } else if (warp == 1 && lane == 0) {
+      constexpr uint32_t idesc = make_idesc_bf16(128, 128, false, false);
       bool ok = mbar_wait(smem_u32(stat_full), 0, p.status, abort_flag) &&
                 mbar_wait(smem_u32(&b_full[0]), 0, p.status, abort_flag);
       if (ok) {
         tc_fence_after();
-        mma_sdp(tmem_base, sA0, sB);
-        mma_sdp(tmem_base + kBt, sA1, sB + kStreamBytes);
-        umma_commit(smem_u32(&sdp_full[0]));
+        mma_tile_128(tmem_base, sA0, false, sB, false, idesc, false);
+        umma_commit(smem_u32(s_full));
+        mma_tile_128(tmem_dp, sA1, false, sB + kTileBytes, false, idesc, false);
+        umma_commit(smem_u32(dp_full));
       }
       for (int i = 0; i < T && ok; ++i) {
-        if (i + 1 < T) {
-          const uint32_t b1 = (i + 1) % kBwdStages, bph1 = ((i + 1) / kBwdStages) & 1, t1 = (i + 1) & 1;
-          if (!mbar_wait(smem_u32(&b_full[b1]), bph1, p.status, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          mma_sdp(tmem_base + t1 * 128, sA0, sB + b1 * 2 * kStreamBytes);
-          mma_sdp(tmem_base + t1 * 128 + kBt, sA1, sB + b1 * 2 * kStreamBytes + kStreamBytes);
-          umma_commit(smem_u32(&sdp_full[t1]));
-        }
-        const uint32_t s = i & 1, ph = (i >> 1) & 1, bsi = i % kBwdStages;
-        if (!mbar_wait(smem_u32(&p_full[s]), ph, p.status, abort_flag)) { ok = false; break; }
+        const uint32_t bs = sB + (i & 1) * 2 * kTileBytes, bn = sB + ((i + 1) & 1) * 2 * kTileBytes;
+        const bool more = i + 1 < T;
+        if (more && !mbar_wait(smem_u32(&b_full[(i + 1) & 1]), ((i + 1) >> 1) & 1, p.status, abort_flag)) { ok = false; break; }
+        if (!mbar_wait(smem_u32(p_ready), i & 1, p.status, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t bs = sB + bsi * 2 * kStreamBytes, ps = sP + s * 2 * kPBytes;
-        if (PT) {
-          if (!DQ) mma_acc_ts(tmem_acc0, tmem_base + s * 128, bs + kStreamBytes, i > 0);
-          mma_acc_ts(tmem_acc1, tmem_base + s * 128 + kBt, bs, i > 0);
-        } else {
-          if (!DQ) mma_acc(tmem_acc0, ps, bs + kStreamBytes, i > 0);     // dV += P^T dO_t
-          mma_acc(tmem_acc1, ps + kPBytes, bs, i > 0);                   // dK += dS^T Q_t   |   dQ += dS K_t
+        // the next S may go over P: the pipe runs one thread's products in the order they were issued
+        if (!DQ) mma_acc_ts(tmem_acc0, tmem_base, bs + kTileBytes, i > 0);             // dV += P^T dO_t
+        if (more) {
+          mma_tile_128(tmem_base, sA0, false, bn, false, idesc, false);
+          umma_commit(smem_u32(s_full));
         }
-        umma_commit(smem_u32(&b_empty[bsi]));
-        umma_commit(smem_u32(&p_free[s]));
+        if (!mbar_wait(smem_u32(ds_ready), i & 1, p.status, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        mma_acc_ts(tmem_acc1, tmem_dp, bs, i > 0);                                     // dK += dS^T Q_t  |  dQ += dS K_t
+        umma_commit(smem_u32(&b_empty[i & 1]));
+        if (more) {
+          mma_tile_128(tmem_dp, sA1, false, bn + kTileBytes, false, idesc, false);
+          umma_commit(smem_u32(dp_full));
+        }
       }
       if (ok) umma_commit(smem_u32(acc_done));
     }
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
     const int q = warp & 3;                      // TMEM lane quadrant this warp may access
-    const int half = (warp - 2) >> 2;            // which 32 of the 64 streamed columns this thread handles
+    const int half = (warp - 4) >> 2;            // which 64 of the 128 streamed columns this thread handles
     const int r = q * 32 + lane;                 // stationary row inside the tile == TMEM lane
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
+    const uint32_t my_s = tmem_base + lane_off + half * 64, my_dp = tmem_dp + lane_off + half * 64;
     const int stat_idx = r0 + r;
-    const long long vec_base = ((long long)b * p.nH + h) * p.S;
-    // DQ: this thread's own row statistics.  Otherwise the streamed rows' statistics go through
-    // shared memory: thread r of the first half fetches lse2 (r < 64) or delta (r >= 64) of streamed row (r & 63).
-    float own_lse = 0.f, own_delta = 0.f;
-    if (DQ && stat_idx < p.S) {
-      own_lse = p.lse2[vec_base + stat_idx];
-      own_delta = p.delta[vec_base + stat_idx];
+    uint64_t own_nlse = 0, own_ndelta = 0;
+    if (DQ) {                                    // the pitch covers whole tiles
+      const float a = p.nlse2[(long long)bh * p.Sp + stat_idx], d = p.ndelta[(long long)bh * p.Sp + stat_idx];
+      own_nlse = pack_f32x2(a, a);
+      own_ndelta = pack_f32x2(d, d);
     }
-    auto fetch = [&](int t) -> float {
-      const int idx = t * kBt + (r & 63);
-      if (DQ || half != 0 || idx >= p.S) return 0.f;
-      return (r < 64) ? p.lse2[vec_base + idx] : p.delta[vec_base + idx];
+    const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2);
+    // zero the elements above the diagonal and past the end of the sequence; first = index of x[0] along the streamed axis
+    auto mask_row = [&](float (&x)[64], int first) {
+#pragma unroll
+      for (int e = 0; e < 64; ++e)
+        if (DQ ? first + e > stat_idx : (first + e < stat_idx || first + e >= p.S)) x[e] = 0.f;
     };
-    float next_val = fetch(t_begin);
-    if (!DQ && half == 0) row_vals[r] = next_val;
     bool ok = true;
     for (int i = 0; i < T; ++i) {
-      const int t = t_begin + i;
-      const uint32_t s = i & 1, ph = (i >> 1) & 1;
-      if (i + 1 < T) next_val = fetch(t + 1);
-      mbar_wait(smem_u32(&sdp_full[s]), ph, p.status, abort_flag);
-      if (!PT && i >= 2) mbar_wait(smem_u32(&p_free[s]), ph ^ 1, p.status, abort_flag);
-      if (softmax_bar_or(*abort_flag != 0)) { ok = false; break; }
+      bool got = mbar_wait(smem_u32(s_full), i & 1, p.status, abort_flag);
+      if (!DQ) got = got && mbar_wait(smem_u32(&b_full[i & 1]), (i >> 1) & 1, p.status, abort_flag);   // the statistics
+      if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
       tc_fence_after();
-      const int c0 = t * kBt;                    // first streamed index of this tile
-      // mask needed when the tile touches the diagonal or the end of the sequence
-      const bool need_mask = DQ ? (c0 + kBt - 1 > r0) : (c0 < r0 + 128 || c0 + kBt > p.S);
-      const float* rv = row_vals + s * 128;
-      uint8_t* prow = smem + AttnBwdSmem::kP + s * 2 * kPBytes + r * 128;
+      const int c0 = (t_begin + i) * 128;        // first streamed index of this tile
+      // tiles on the diagonal and at the end of the sequence have elements that do not count
+      const bool need_mask = c0 == r0 || (!DQ && c0 + 128 > p.S);
+      const uint64_t* rv = reinterpret_cast<const uint64_t*>(smem + AttnBwdSmem::kRow + (i & 1) * 2 * kStatBytes) + half * 32;
+      float pe[64];
       {
-        const int c = half;
-        uint32_t sv[32], dv[32];
-        tmem_ld_32x32b_x32(tmem_base + s * 128 + lane_off + c * 32, sv);
-        tmem_ld_32x32b_x32(tmem_base + s * 128 + kBt + lane_off + c * 32, dv);
+        uint32_t sv[64];
+        tmem_ld_32x32b_x32(my_s, *reinterpret_cast<uint32_t(*)[32]>(sv));
+        tmem_ld_32x32b_x32(my_s + 32, *reinterpret_cast<uint32_t(*)[32]>(sv + 32));
         tmem_ld_wait();
-        uint32_t pp[16], dd[16];
 #pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          float l4[4], d4[4];
-          if (DQ) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) { l4[u] = own_lse; d4[u] = own_delta; }
-          } else {
-            const float4 a = *reinterpret_cast<const float4*>(rv + c * 32 + e);
-            const float4 bq = *reinterpret_cast<const float4*>(rv + 64 + c * 32 + e);
-            l4[0] = a.x; l4[1] = a.y; l4[2] = a.z; l4[3] = a.w;
-            d4[0] = bq.x; d4[1] = bq.y; d4[2] = bq.z; d4[3] = bq.w;
-          }
-          float pv[4], dsv[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            float pe = exp2f(__uint_as_float(sv[e + u]) * p.scale_log2 - l4[u]);
-            float de = pe * (__uint_as_float(dv[e + u]) - d4[u]) * p.scale;
-            if (need_mask) {
-              const int sidx = c0 + c * 32 + e + u;
-              const bool valid = DQ ? (sidx <= stat_idx) : (sidx >= stat_idx && sidx < p.S);
-              if (!valid) { pe = 0.f; de = 0.f; }
-            }
-            pv[u] = pe; dsv[u] = de;
-          }
-          pp[e >> 1] = pack_bf16x2(pv[0], pv[1]);
-          pp[(e >> 1) + 1] = pack_bf16x2(pv[2], pv[3]);
-          dd[e >> 1] = pack_bf16x2(dsv[0], dsv[1]);
-          dd[(e >> 1) + 1] = pack_bf16x2(dsv[2], dsv[3]);
-        }
-        if (PT) {
-          // over the columns this thread just read: P at the start of its 32 S columns, dS likewise in dP
-          if (!DQ) tmem_st_32x32b_x16(tmem_base + s * 128 + lane_off + c * 32, pp);
-          tmem_st_32x32b_x16(tmem_base + s * 128 + kBt + lane_off + c * 32, dd);
-          tmem_st_wait();
-        } else {
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            const int phys = ((c * 4 + g) ^ (r & 7)) * 16;
-            if (!DQ) *reinterpret_cast<uint4*>(prow + phys) = make_uint4(pp[g * 4], pp[g * 4 + 1], pp[g * 4 + 2], pp[g * 4 + 3]);
-            *reinterpret_cast<uint4*>(prow + kPBytes + phys) = make_uint4(dd[g * 4], dd[g * 4 + 1], dd[g * 4 + 2], dd[g * 4 + 3]);
-          }
+        for (int e = 0; e < 32; ++e) {
+          unpack_f32x2(fma_f32x2(pack_u32x2(sv[2 * e], sv[2 * e + 1]), sc2, DQ ? own_nlse : rv[e]), pe[2 * e], pe[2 * e + 1]);
+          pe[2 * e] = exp2f(pe[2 * e]);
+          pe[2 * e + 1] = exp2f(pe[2 * e + 1]);
         }
       }
-      if (!DQ && half == 0 && i + 1 < T) row_vals[(s ^ 1) * 128 + r] = next_val;
-      if (!PT) fence_proxy_async_smem();
+      if (need_mask) mask_row(pe, c0 + half * 64);
+      if (!DQ) {
+        uint32_t pk[32];
+#pragma unroll
+        for (int e = 0; e < 32; ++e) pk[e] = pack_bf16x2(pe[2 * e], pe[2 * e + 1]);
+        tmem_st_32x32b_x32(my_s, pk);
+        tmem_st_wait();
+      }
       tc_fence_before();
-      mbar_arrive(smem_u32(&p_full[s]));
+      mbar_arrive(smem_u32(p_ready));
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(dp_full), i & 1, p.status, abort_flag))) { ok = false; break; }
+      tc_fence_after();
+      {
+        uint32_t dv[64], pk[32];
+        tmem_ld_32x32b_x32(my_dp, *reinterpret_cast<uint32_t(*)[32]>(dv));
+        tmem_ld_32x32b_x32(my_dp + 32, *reinterpret_cast<uint32_t(*)[32]>(dv + 32));
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 32; ++e)
+          unpack_f32x2(mul_f32x2(pack_f32x2(pe[2 * e], pe[2 * e + 1]),
+                                 add_f32x2(pack_u32x2(dv[2 * e], dv[2 * e + 1]), DQ ? own_ndelta : rv[64 + e])),
+                       pe[2 * e], pe[2 * e + 1]);
+        if (need_mask) mask_row(pe, c0 + half * 64);         // 0 * inf from elements that do not count
+#pragma unroll
+        for (int e = 0; e < 32; ++e) pk[e] = pack_bf16x2(pe[2 * e], pe[2 * e + 1]);
+        tmem_st_32x32b_x32(my_dp, pk);
+        tmem_st_wait();
+      }
+      tc_fence_before();
+      mbar_arrive(smem_u32(ds_ready));
     }
-    if (ok) {
-      mbar_wait(smem_u32(acc_done), 0, p.status, abort_flag);
-      ok = !softmax_bar_or(*abort_flag != 0);
-    }
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc_done), 0, p.status, abort_flag));
     if (ok) {
       // tcgen05.ld is warp-collective: every lane takes part, only the stores depend on the row being valid
       const bool row_ok = stat_idx < p.S;
@@ -828,8 +782,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_consta
       __nv_bfloat16* grow = p.dqkv + (long long)(row_base + stat_idx) * p.ld_dqkv + h * kHd;
 #pragma unroll
       for (int a = (DQ ? 1 : 0); a < 2; ++a) {
-        // acc0 = dV (columns 2H..), acc1 = dK (columns H..) or dQ (columns 0..); each half stores 64 columns
+        // acc0 = dV (columns 2H..); acc1 = dK (columns H..) or dQ (columns 0..), whose factor is applied here, once,
+        // to the fp32 sums; each half stores 64 columns
         __nv_bfloat16* dst = grow + (DQ ? 0 : (a == 0 ? 2 * H : H)) + half * 64;
+        const float f = a == 0 ? 1.f : p.scale;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           uint32_t t4[32];
@@ -839,10 +795,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_consta
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
             uint4 o;
-            o.x = pack_bf16x2(__uint_as_float(t4[g * 8 + 0]), __uint_as_float(t4[g * 8 + 1]));
-            o.y = pack_bf16x2(__uint_as_float(t4[g * 8 + 2]), __uint_as_float(t4[g * 8 + 3]));
-            o.z = pack_bf16x2(__uint_as_float(t4[g * 8 + 4]), __uint_as_float(t4[g * 8 + 5]));
-            o.w = pack_bf16x2(__uint_as_float(t4[g * 8 + 6]), __uint_as_float(t4[g * 8 + 7]));
+            o.x = pack_bf16x2(__uint_as_float(t4[g * 8 + 0]) * f, __uint_as_float(t4[g * 8 + 1]) * f);
+            o.y = pack_bf16x2(__uint_as_float(t4[g * 8 + 2]) * f, __uint_as_float(t4[g * 8 + 3]) * f);
+            o.z = pack_bf16x2(__uint_as_float(t4[g * 8 + 4]) * f, __uint_as_float(t4[g * 8 + 5]) * f);
+            o.w = pack_bf16x2(__uint_as_float(t4[g * 8 + 6]) * f, __uint_as_float(t4[g * 8 + 7]) * f);
             *reinterpret_cast<uint4*>(dst + c * 32 + g * 8) = o;
           }
         }
@@ -858,28 +814,37 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_consta
   }
 }
 
-// lse2 = lse * log2(e); delta = rowsum(dO * O).  One warp per (row, head).
-__global__ void attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ dout, long long ld_do,
-                                     const __nv_bfloat16* __restrict__ out, long long ld_o,
-                                     const float* __restrict__ lse, float* __restrict__ lse2,
-                                     float* __restrict__ delta, int B, int S, int nH) {
-  const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  const long long total = (long long)B * S * nH;
-  if (w >= total) return;
+// nlse2 = -lse * log2(e); ndelta = -rowsum(dO * O); both zero for the rows that pad a head to whole tiles.  Half a
+// warp per (row, head), 16 bytes of each operand per lane.
+__global__ void __launch_bounds__(256)
+attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ dout, long long ld_do, const __nv_bfloat16* __restrict__ out,
+                     long long ld_o, const float* __restrict__ lse, float* __restrict__ nlse2, float* __restrict__ ndelta,
+                     int B, int S, int nH, int Sp) {
+  const long long w = (long long)blockIdx.x * 16 + (threadIdx.x >> 4);
+  const int lane = threadIdx.x & 15;
+  if (w >= (long long)B * Sp * nH) return;                 // whole half-warps leave
   const int hh = (int)(w % nH);
   const long long row = w / nH;
-  const int bb = (int)(row / S), ss = (int)(row % S);
-  const uint2 a = *reinterpret_cast<const uint2*>(dout + row * ld_do + hh * kHd + lane * 4);
-  const uint2 o = *reinterpret_cast<const uint2*>(out + row * ld_o + hh * kHd + lane * 4);
-  const float2 a0 = unpack_bf16x2(a.x), a1 = unpack_bf16x2(a.y), o0 = unpack_bf16x2(o.x), o1 = unpack_bf16x2(o.y);
-  float acc = a0.x * o0.x + a0.y * o0.y + a1.x * o1.x + a1.y * o1.y;
+  const int bb = (int)(row / Sp), ss = (int)(row % Sp);
+  float acc = 0.f;
+  if (ss < S) {
+    const long long t = (long long)bb * S + ss;
+    const uint4 a = *reinterpret_cast<const uint4*>(dout + t * ld_do + hh * kHd + lane * 8);
+    const uint4 o = *reinterpret_cast<const uint4*>(out + t * ld_o + hh * kHd + lane * 8);
+    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, ow[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    for (int e = 0; e < 4; ++e) {
+      const float2 x = unpack_bf16x2(aw[e]), y = unpack_bf16x2(ow[e]);
+      acc += x.x * y.x + x.y * y.y;
+    }
+  }
+  const unsigned mask = 0xffffu << (threadIdx.x & 16);
+#pragma unroll
+  for (int off = 8; off > 0; off >>= 1) acc += __shfl_xor_sync(mask, acc, off);
   if (lane == 0) {
-    const long long idx = ((long long)bb * nH + hh) * S + ss;
-    delta[idx] = acc;
-    lse2[idx] = lse[idx] * kLog2e;
+    const long long head = (long long)bb * nH + hh, idx = head * Sp + ss;
+    ndelta[idx] = -acc;
+    nlse2[idx] = ss < S ? -lse[head * S + ss] * kLog2e : 0.f;
   }
 }
 }  // namespace mfsdp
@@ -888,6 +853,10 @@ using namespace mfsdp;
 
 // Bytes of K and V that a group of heads may occupy (half of the 126 MB L2, the rest is for Q, O and the other die).
 constexpr long long kKvInL2 = 64LL << 20;
+static int heads_in_l2(int B, int S, int nH) {
+  const long long group = kKvInL2 / ((long long)S * kHd * 2 * 2), heads = (long long)B * nH;
+  return (int)(group < 1 ? 1 : group > heads ? heads : group);
+}
 
 // A grid of at most one 128-query tile per SM is as long as its longest tile, which two threads per row finish sooner
 // (16 heads of 1024 rows: 20 us in one-tile blocks, 25 in two); above that two tiles per block win at every size tried.
@@ -917,10 +886,7 @@ MFSDP_API int mfsdp_attention_fwd(const void* qkv, void* out, float* lse, int B,
   a.out = (__nv_bfloat16*)out; a.ld_out = ld_out; a.lse = lse; a.status = status;
   if (attn_fwd_two_tiles(B, S, nH)) {
     const int nq = (S + 2 * kBq - 1) / (2 * kBq);
-    long long group = kKvInL2 / ((long long)S * kHd * 2 * 2);
-    if (group < 1) group = 1;
-    if (group > (long long)B * nH) group = (long long)B * nH;
-    attn_fwd2_kernel<<<(unsigned)(nq * B * nH), kFwd2Threads, AttnFwd2Smem::kBytes, st>>>(map, a, (int)group);
+    attn_fwd2_kernel<<<(unsigned)(nq * B * nH), kFwd2Threads, AttnFwd2Smem::kBytes, st>>>(map, a, heads_in_l2(B, S, nH));
     return (int)cudaGetLastError();
   }
   dim3 grid((S + kBq - 1) / kBq, nH, B);
@@ -929,48 +895,39 @@ MFSDP_API int mfsdp_attention_fwd(const void* qkv, void* out, float* lse, int B,
 }
 
 // dout, out: [B*S, nH*128] bf16; lse: [B, nH, S]; dqkv: [B*S, 3*nH*128] bf16 (written in full);
-// scratch: 2 * B * nH * S floats.
+// scratch: 2 * B * nH * Sp floats, 16-byte aligned, Sp = S rounded up to 128.
 MFSDP_API int mfsdp_attention_bwd(const void* dout, const void* qkv, const void* out, const float* lse, void* dqkv,
                                   float* scratch, int B, int S, int nH, long long ld_qkv, long long ld_o,
                                   long long ld_dqkv, float softmax_scale, int* status, cudaStream_t st) {
-  if (B <= 0 || S <= 0 || nH <= 0 || (ld_qkv % 8) || (ld_o % 8) || (ld_dqkv % 8) || !scratch) return -2;
+  if (B <= 0 || S <= 0 || nH <= 0 || (ld_qkv % 8) || (ld_o % 8) || (ld_dqkv % 8) || !scratch || ((uintptr_t)scratch & 15)) return -2;
   ensure_context_on_this_thread();
   CUtensorMap map_qkv, map_do;
-  int rc = make_tmap_bf16_2d(&map_qkv, qkv, (long long)B * S, 3LL * nH * kHd, ld_qkv, kBt, 64);
+  int rc = make_tmap_bf16_2d(&map_qkv, qkv, (long long)B * S, 3LL * nH * kHd, ld_qkv, 128, 64);
   if (rc) return rc;
-  rc = make_tmap_bf16_2d(&map_do, dout, (long long)B * S, (long long)nH * kHd, ld_o, kBt, 64);
+  rc = make_tmap_bf16_2d(&map_do, dout, (long long)B * S, (long long)nH * kHd, ld_o, 128, 64);
   if (rc) return rc;
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaSuccess;
-    const void* kerns[4] = {(const void*)attn_bwd_kernel<false, false>, (const void*)attn_bwd_kernel<true, false>,
-                            (const void*)attn_bwd_kernel<false, true>, (const void*)attn_bwd_kernel<true, true>};
-    for (int i = 0; i < 4 && e == cudaSuccess; ++i)
-      e = cudaFuncSetAttribute(kerns[i], cudaFuncAttributeMaxDynamicSharedMemorySize, AttnBwdSmem::kBytes);
+    cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnBwdSmem::kBytes);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(attn_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnBwdSmem::kBytes);
     if (e != cudaSuccess) return (int)e;
     attr = true;
   }
-  const long long n = (long long)B * nH * S;
-  float* lse2 = scratch;
-  float* delta = scratch + n;
-  attn_bwd_prep_kernel<<<(unsigned)((n + 7) / 8), 256, 0, st>>>((const __nv_bfloat16*)dout, ld_o, (const __nv_bfloat16*)out,
-                                                                ld_o, lse, lse2, delta, B, S, nH);
+  const int nt = (S + 127) / 128;
   AttnBwdArgs a{};
   a.B = B; a.S = S; a.nH = nH;
+  a.Sp = (long long)nt * 128;
+  float* nlse2 = scratch;
+  float* ndelta = scratch + (long long)B * nH * a.Sp;
+  attn_bwd_prep_kernel<<<(unsigned)(((long long)B * nH * a.Sp + 15) / 16), 256, 0, st>>>(
+      (const __nv_bfloat16*)dout, ld_o, (const __nv_bfloat16*)out, ld_o, lse, nlse2, ndelta, B, S, nH, (int)a.Sp);
   a.scale = softmax_scale; a.scale_log2 = softmax_scale * kLog2e;
-  a.lse2 = lse2; a.delta = delta;
+  a.nlse2 = nlse2; a.ndelta = ndelta;
   a.dqkv = (__nv_bfloat16*)dqkv; a.ld_dqkv = ld_dqkv; a.status = status;
-  dim3 grid((S + 127) / 128, nH, B);
-  static const bool p_in_tmem = [] {
-    const char* e = getenv("MFSDP_ATTN_P_TMEM");
-    return e ? atoi(e) != 0 : true;
-  }();
-  if (p_in_tmem) {
-    attn_bwd_kernel<false, true><<<grid, kAttnThreads, AttnBwdSmem::kBytes, st>>>(map_qkv, map_do, a);
-    attn_bwd_kernel<true, true><<<grid, kAttnThreads, AttnBwdSmem::kBytes, st>>>(map_qkv, map_do, a);
-  } else {
-    attn_bwd_kernel<false, false><<<grid, kAttnThreads, AttnBwdSmem::kBytes, st>>>(map_qkv, map_do, a);
-    attn_bwd_kernel<true, false><<<grid, kAttnThreads, AttnBwdSmem::kBytes, st>>>(map_qkv, map_do, a);
-  }
+  a.heads_per_group = heads_in_l2(B, S, nH);
+  const unsigned grid = (unsigned)(nt * B * nH);
+  attn_bwd_kernel<false><<<grid, kBwdThreads, AttnBwdSmem::kBytes, st>>>(map_qkv, map_do, a);
+  attn_bwd_kernel<true><<<grid, kBwdThreads, AttnBwdSmem::kBytes, st>>>(map_qkv, map_do, a);
   return (int)cudaGetLastError();
 }

@@ -117,3 +117,33 @@ def test_attention_fwd_two_tiles_rescale():
     ref_o, ref_lse = _ref(qkv, B, S, nH, hd)
     assert (out.float() - ref_o).abs().max().item() < 4e-2
     assert (lse - ref_lse).abs().max().item() < 5e-3
+
+
+@pytest.mark.parametrize("B,S,nH,heads", [(1, 1, 3, (0, 2)), (2, 127, 2, (0, 1)), (1, 129, 2, (1,)), (2, 1000, 3, (0, 2)),
+                                          (1, 8192, 17, (0, 15, 16))])
+def test_attention_bwd_tiles_and_head_groups(B, S, nH, heads):
+    """One row, both sides of a tile edge, batches whose last tile reads the next one's rows, and more heads than one
+    group of the block order.  Bound: bf16 inputs, P and dS of products with fp32 sums, 1e-2 in the 2-norm."""
+    from matrix_fsdp_b200.ops import attention as A
+    from matrix_fsdp_b200.ops import kernels as K
+
+    torch.manual_seed(2)
+    hd = 128
+    qkv = torch.randn(B * S, 3 * nH * hd, device="cuda", dtype=torch.bfloat16)
+    dout = torch.randn(B * S, nH * hd, device="cuda", dtype=torch.bfloat16)
+    out, lse = A.attention_fwd(qkv, B, S, nH, hd)
+    dqkv = A.attention_bwd(dout, qkv, out, lse, B, S, nH, hd)
+    K.check_status()
+    assert torch.isfinite(dqkv).all()
+    for b in range(B):
+        for h in heads:
+            cols = [slice((i * nH + h) * hd, (i * nH + h + 1) * hd) for i in range(3)]
+            one = torch.cat([qkv[b * S:(b + 1) * S, c] for c in cols], dim=1).float().requires_grad_(True)
+            ref_o, _ = _ref(one, 1, S, 1, hd)
+            (ref,) = torch.autograd.grad(ref_o, one, dout[b * S:(b + 1) * S, h * hd:(h + 1) * hd].float())
+            got = torch.cat([dqkv[b * S:(b + 1) * S, c] for c in cols], dim=1).float()
+            for i in range(3):
+                g, w = got[:, i * hd:(i + 1) * hd], ref[:, i * hd:(i + 1) * hd]
+                # with one row P is 1 and dS cancels: the rounding of dO and O remains, 2^-8 of their products
+                floor = 2 ** -7 * one[:, :].norm() if S == 1 else 0.0
+                assert (g - w).norm() <= 1e-2 * w.norm() + floor, (b, h, i)
