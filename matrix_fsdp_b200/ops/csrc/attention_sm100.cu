@@ -539,7 +539,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs 
 // Two kernels without atomics (the sums have one order in every run), sharing one body:
 //   DQ = false: one CTA per (batch, head, 128-key tile).  K_j and V_j stay in shared memory, the query axis streams
 //               in tiles of 128 rows (Q_i, dO_i).  S^T = K_j Q_i^T and dP^T = V_j dO_i^T land in TMEM (thread = key
-//               row, two threads per row), P^T and dS^T go back over them as bf16, dV += P^T dO_i and dK += dS^T Q_i
+//               row, four threads per row), P^T and dS^T go back over them as bf16, dV += P^T dO_i and dK += dS^T Q_i
 //               accumulate in TMEM.
 //   DQ = true : one CTA per (batch, head, 128-query tile).  Q_i and dO_i stay, keys stream (K_j, V_j).
 //               S = Q_i K_j^T, dP = dO_i V_j^T, dQ += dS K_j.
@@ -547,8 +547,18 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs 
 // dry although every buffer is single: while the threads turn dP into dS the pipe adds to dV and computes the next S,
 // and while they take exponentials of that S it adds to dK / dQ and computes the next dP.  128-wide streamed tiles,
 // because a 64-wide second operand makes the products wait for shared memory (A and B together 192 B per cycle).
-// The row statistics of a streamed tile arrive with it, in the same barrier, so no thread waits for another.
-constexpr int kBwdThreads = 384;      // warp 0 TMA, warp 1 MMA, 2 and 3 idle, warps 4-11 P and dS
+// Streamed tiles go through a ring of five 32 KB buffers in the order of their first use (Q_0 dO_0 Q_1 dO_1 Q_2 ... |
+// K_0 V_0 K_1 ...), each freed by the last product that reads it: with two buffers per operand a load could only start
+// one product before its tile was needed, and the pipe was busy 43 % of the time.  The row statistics of a streamed tile
+// arrive with it, in the same barriers, so no thread waits for another.
+// Four threads share a row: with two (2 warps per scheduler) the fixed latencies of the element-wise chains showed.
+// Measured (64-wide streamed tiles -> 128-wide in pairs of buffers -> this): 16 heads of 2 x 4096 rows 806 -> 547 ->
+// 503 us, 32 heads of 16384 rows 10.1 -> 7.2 -> 6.4 ms (857 TFLOP/s counting five products per tile), 16 heads of
+// 3 x 1333 rows 205 -> 157 -> 152 us.
+constexpr int kBwdThreads = 640;      // warp 0 TMA, warp 1 MMA, 2 and 3 idle, warps 4-19 P and dS
+constexpr int kBwdCols = 32;          // streamed columns per thread
+// 640 threads are launched with 96 registers each, 61,440 in all: 128 * 64 + 512 * 104.
+constexpr int kBwdRegsIssue = 64, kBwdRegsSoftmax = 104;
 constexpr int kStatBytes = 128 * 4;   // one row statistic of a streamed tile
 
 struct AttnBwdArgs {
@@ -563,23 +573,26 @@ struct AttnBwdArgs {
   int heads_per_group;
 };
 
+constexpr int kRing = 5;
 struct AttnBwdSmem {
   static constexpr int kA0 = 0;
   static constexpr int kA1 = kA0 + kTileBytes;
-  static constexpr int kB = kA1 + kTileBytes;             // 2 stages x (B0, B1)
-  static constexpr int kRow = kB + 4 * kTileBytes;        // 2 stages x (nlse2, ndelta)
-  static constexpr int kBars = kRow + 4 * kStatBytes;
-  static constexpr int kBytes = kBars + 256 + 1024;
+  static constexpr int kB = kA1 + kTileBytes;             // the ring
+  static constexpr int kNlse = kB + kRing * kTileBytes;   // 3 stages: a tile's Q is loaded while two earlier S wait
+  static constexpr int kNdelta = kNlse + 3 * kStatBytes;  // 2 stages
+  static constexpr int kBars = kNdelta + 2 * kStatBytes;
+  static constexpr int kBytes = kBars + 256;              // 232,192 of the 232,448 that a block may have
 };
 
-// D[128 x 128] (+)= P[128 x 128] * B[128 rows along K x 128, N contiguous].  The two threads of a row have each packed
-// their 64 elements into the first 32 columns of their own half.
+
+// D[128 x 128] (+)= P[128 x 128] * B[128 rows along K x 128, N contiguous].  The four threads of a row have each packed
+// their 32 elements into the first 16 columns of their own quarter.
 __device__ __forceinline__ void mma_acc_ts(uint32_t tmem_d, uint32_t tmem_p, uint32_t b_base, bool accumulate) {
   constexpr uint32_t idesc = make_idesc_bf16(128, 128, false, true);
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const uint64_t bd = make_smem_desc_sw128(b_base + k * 2048, kHalfTile, 1024);
-    umma_f16_ts(tmem_d, tmem_p + (k >> 2) * 64 + (k & 3) * 8, bd, idesc, (accumulate || k > 0) ? 1u : 0u);
+    umma_f16_ts(tmem_d, tmem_p + (k >> 1) * 32 + (k & 1) * 8, bd, idesc, (accumulate || k > 0) ? 1u : 0u);
   }
 }
 
@@ -587,18 +600,21 @@ template <bool DQ>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_constant__ CUtensorMap tma_do,
                 const AttnBwdArgs p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if (smem_u32(smem) & 1023) {         // the swizzled tiles need it; nothing has been started yet
+    if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, (int)kErrBadArgument);
+    return;
+  }
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + AttnBwdSmem::kBars);
-  uint64_t* stat_full = bars;          // [1]
-  uint64_t* b_full = bars + 1;         // [2]
-  uint64_t* b_empty = bars + 3;        // [2] all products of a streamed tile have finished
-  uint64_t* s_full = bars + 5;         // [1]
-  uint64_t* dp_full = bars + 6;        // [1]
-  uint64_t* p_ready = bars + 7;        // [1] count 256: S read, P written
-  uint64_t* ds_ready = bars + 8;       // [1] count 256: dP read, dS written
-  uint64_t* acc_done = bars + 9;       // [1]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+  uint64_t* full = bars;               // [5] ring: tile 2i is Q_i / K_i, tile 2i+1 is dO_i / V_i
+  uint64_t* empty = bars + kRing;      // [5] the last product that reads a tile has finished
+  uint64_t* stat_full = bars + 10;     // [1]
+  uint64_t* s_full = bars + 11;        // [1]
+  uint64_t* dp_full = bars + 12;       // [1]
+  uint64_t* p_ready = bars + 13;       // [1] count 512: S read, P written
+  uint64_t* ds_ready = bars + 14;      // [1] count 512: dP read, dS written
+  uint64_t* acc_done = bars + 15;      // [1]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -621,7 +637,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_consta
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    for (int i = 0; i < 10; ++i) mbar_init(smem_u32(&bars[i]), (i == 7 || i == 8) ? 256 : 1);
+    for (int i = 0; i < 16; ++i) mbar_init(smem_u32(&bars[i]), (i == 13 || i == 14) ? 512 : 1);
     mbar_fence_init();
     tma_prefetch_desc(&tma_qkv);
     tma_prefetch_desc(&tma_do);
@@ -636,10 +652,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_dp = tmem_base + 128, tmem_acc0 = tmem_base + 256, tmem_acc1 = tmem_base + 384;
   const uint32_t sA0 = smem_u32(smem + AttnBwdSmem::kA0), sA1 = smem_u32(smem + AttnBwdSmem::kA1),
-                 sB = smem_u32(smem + AttnBwdSmem::kB), sRow = smem_u32(smem + AttnBwdSmem::kRow);
+                 sB = smem_u32(smem + AttnBwdSmem::kB);
+  auto slot = [&](int tile_idx) { return sB + (uint32_t)(tile_idx % kRing) * kTileBytes; };
+  auto full_bar = [&](int tile_idx) { return smem_u32(&full[tile_idx % kRing]); };
+  auto full_phase = [&](int tile_idx) { return (uint32_t)(tile_idx / kRing) & 1u; };
 
   if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kBwdRegsIssue));
     if (warp == 0 && lane == 0) {
       mbar_arrive_expect_tx(smem_u32(stat_full), 2 * kTileBytes);
       if (DQ) {
@@ -649,63 +668,73 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_consta
         tma_load_tile(sA0, &tma_qkv, smem_u32(stat_full), H + h * kHd, row_base + r0);      // K_j
         tma_load_tile(sA1, &tma_qkv, smem_u32(stat_full), 2 * H + h * kHd, row_base + r0);  // V_j
       }
-      for (int i = 0; i < T; ++i) {
-        const uint32_t s = i & 1, ph = (i >> 1) & 1;
-        if (!mbar_wait(smem_u32(&b_empty[s]), ph ^ 1, p.status, abort_flag)) break;
-        const uint32_t bar = smem_u32(&b_full[s]), dst = sB + s * 2 * kTileBytes;
-        mbar_arrive_expect_tx(bar, 2 * kTileBytes + (DQ ? 0 : 2 * kStatBytes));
-        const int t0 = (t_begin + i) * 128, row = row_base + t0;
+      for (int k = 0; k < 2 * T; ++k) {
+        if (!mbar_wait(smem_u32(&empty[k % kRing]), full_phase(k) ^ 1, p.status, abort_flag)) break;
+        const uint32_t bar = full_bar(k);
+        mbar_arrive_expect_tx(bar, kTileBytes + (DQ ? 0 : kStatBytes));
+        const int i = k >> 1, t0 = (t_begin + i) * 128, row = row_base + t0;
+        const long long stat = (long long)bh * p.Sp + t0;
         if (DQ) {
-          tma_load_tile(dst, &tma_qkv, bar, H + h * kHd, row);                       // K_t
-          tma_load_tile(dst + kTileBytes, &tma_qkv, bar, 2 * H + h * kHd, row);      // V_t
+          tma_load_tile(slot(k), &tma_qkv, bar, ((k & 1) ? 2 * H : H) + h * kHd, row);          // K_t, V_t
+        } else if (k & 1) {
+          tma_load_tile(slot(k), &tma_do, bar, h * kHd, row);                                   // dO_t
+          bulk_load(smem_u32(smem + AttnBwdSmem::kNdelta + (i & 1) * kStatBytes), p.ndelta + stat, kStatBytes, bar);
         } else {
-          tma_load_tile(dst, &tma_qkv, bar, h * kHd, row);                           // Q_t
-          tma_load_tile(dst + kTileBytes, &tma_do, bar, h * kHd, row);               // dO_t
-          bulk_load(sRow + s * 2 * kStatBytes, p.nlse2 + (long long)bh * p.Sp + t0, kStatBytes, bar);
-          bulk_load(sRow + s * 2 * kStatBytes + kStatBytes, p.ndelta + (long long)bh * p.Sp + t0, kStatBytes, bar);
+          tma_load_tile(slot(k), &tma_qkv, bar, h * kHd, row);                                  // Q_t
+          bulk_load(smem_u32(smem + AttnBwdSmem::kNlse + (i % 3) * kStatBytes), p.nlse2 + stat, kStatBytes, bar);
         }
       }
     } else if (warp == 1 && lane == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(128, 128, false, false);
-      bool ok = mbar_wait(smem_u32(stat_full), 0, p.status, abort_flag) &&
-                mbar_wait(smem_u32(&b_full[0]), 0, p.status, abort_flag);
+      bool ok = mbar_wait(smem_u32(stat_full), 0, p.status, abort_flag) && mbar_wait(full_bar(0), 0, p.status, abort_flag);
       if (ok) {
         tc_fence_after();
-        mma_tile_128(tmem_base, sA0, false, sB, false, idesc, false);
+        mma_tile_128(tmem_base, sA0, false, slot(0), false, idesc, false);
         umma_commit(smem_u32(s_full));
-        mma_tile_128(tmem_dp, sA1, false, sB + kTileBytes, false, idesc, false);
+        ok = mbar_wait(full_bar(1), 0, p.status, abort_flag);
+      }
+      if (ok) {
+        tc_fence_after();
+        mma_tile_128(tmem_dp, sA1, false, slot(1), false, idesc, false);
         umma_commit(smem_u32(dp_full));
+        if (DQ) umma_commit(smem_u32(&empty[1]));                                      // V_0 is not read again
       }
       for (int i = 0; i < T && ok; ++i) {
-        const uint32_t bs = sB + (i & 1) * 2 * kTileBytes, bn = sB + ((i + 1) & 1) * 2 * kTileBytes;
+        const int k = 2 * i;
         const bool more = i + 1 < T;
-        if (more && !mbar_wait(smem_u32(&b_full[(i + 1) & 1]), ((i + 1) >> 1) & 1, p.status, abort_flag)) { ok = false; break; }
+        if (more && !mbar_wait(full_bar(k + 2), full_phase(k + 2), p.status, abort_flag)) { ok = false; break; }
         if (!mbar_wait(smem_u32(p_ready), i & 1, p.status, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        // the next S may go over P: the pipe runs one thread's products in the order they were issued
-        if (!DQ) mma_acc_ts(tmem_acc0, tmem_base, bs + kTileBytes, i > 0);             // dV += P^T dO_t
+        if (!DQ) {
+          mma_acc_ts(tmem_acc0, tmem_base, slot(k + 1), i > 0);                        // dV += P^T dO_t
+          umma_commit(smem_u32(&empty[(k + 1) % kRing]));
+        }
         if (more) {
-          mma_tile_128(tmem_base, sA0, false, bn, false, idesc, false);
+          // the next S may go over P: the pipe runs one thread's products in the order they were issued
+          mma_tile_128(tmem_base, sA0, false, slot(k + 2), false, idesc, false);
           umma_commit(smem_u32(s_full));
         }
         if (!mbar_wait(smem_u32(ds_ready), i & 1, p.status, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        mma_acc_ts(tmem_acc1, tmem_dp, bs, i > 0);                                     // dK += dS^T Q_t  |  dQ += dS K_t
-        umma_commit(smem_u32(&b_empty[i & 1]));
+        mma_acc_ts(tmem_acc1, tmem_dp, slot(k), i > 0);                                // dK += dS^T Q_t  |  dQ += dS K_t
+        umma_commit(smem_u32(&empty[k % kRing]));
         if (more) {
-          mma_tile_128(tmem_dp, sA1, false, bn + kTileBytes, false, idesc, false);
+          if (!mbar_wait(full_bar(k + 3), full_phase(k + 3), p.status, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          mma_tile_128(tmem_dp, sA1, false, slot(k + 3), false, idesc, false);
           umma_commit(smem_u32(dp_full));
+          if (DQ) umma_commit(smem_u32(&empty[(k + 3) % kRing]));
         }
       }
       if (ok) umma_commit(smem_u32(acc_done));
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kBwdRegsSoftmax));
     const int q = warp & 3;                      // TMEM lane quadrant this warp may access
-    const int half = (warp - 4) >> 2;            // which 64 of the 128 streamed columns this thread handles
+    const int part = (warp - 4) >> 2;            // which 32 of the 128 streamed columns this thread handles
     const int r = q * 32 + lane;                 // stationary row inside the tile == TMEM lane
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
-    const uint32_t my_s = tmem_base + lane_off + half * 64, my_dp = tmem_dp + lane_off + half * 64;
+    const uint32_t my_s = tmem_base + lane_off + part * kBwdCols, my_dp = tmem_dp + lane_off + part * kBwdCols;
     const int stat_idx = r0 + r;
     uint64_t own_nlse = 0, own_ndelta = 0;
     if (DQ) {                                    // the pitch covers whole tiles
@@ -715,60 +744,61 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_consta
     }
     const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2);
     // zero the elements above the diagonal and past the end of the sequence; first = index of x[0] along the streamed axis
-    auto mask_row = [&](float (&x)[64], int first) {
+    auto mask_row = [&](float (&x)[kBwdCols], int first) {
 #pragma unroll
-      for (int e = 0; e < 64; ++e)
+      for (int e = 0; e < kBwdCols; ++e)
         if (DQ ? first + e > stat_idx : (first + e < stat_idx || first + e >= p.S)) x[e] = 0.f;
     };
     bool ok = true;
     for (int i = 0; i < T; ++i) {
       bool got = mbar_wait(smem_u32(s_full), i & 1, p.status, abort_flag);
-      if (!DQ) got = got && mbar_wait(smem_u32(&b_full[i & 1]), (i >> 1) & 1, p.status, abort_flag);   // the statistics
+      if (!DQ) got = got && mbar_wait(full_bar(2 * i), full_phase(2 * i), p.status, abort_flag);   // nlse2
       if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
       tc_fence_after();
       const int c0 = (t_begin + i) * 128;        // first streamed index of this tile
       // tiles on the diagonal and at the end of the sequence have elements that do not count
       const bool need_mask = c0 == r0 || (!DQ && c0 + 128 > p.S);
-      const uint64_t* rv = reinterpret_cast<const uint64_t*>(smem + AttnBwdSmem::kRow + (i & 1) * 2 * kStatBytes) + half * 32;
-      float pe[64];
+      const uint64_t* nlse = reinterpret_cast<const uint64_t*>(smem + AttnBwdSmem::kNlse + (i % 3) * kStatBytes) + part * (kBwdCols / 2);
+      const uint64_t* ndelta = reinterpret_cast<const uint64_t*>(smem + AttnBwdSmem::kNdelta + (i & 1) * kStatBytes) + part * (kBwdCols / 2);
+      float pe[kBwdCols];
       {
-        uint32_t sv[64];
-        tmem_ld_32x32b_x32(my_s, *reinterpret_cast<uint32_t(*)[32]>(sv));
-        tmem_ld_32x32b_x32(my_s + 32, *reinterpret_cast<uint32_t(*)[32]>(sv + 32));
+        uint32_t sv[kBwdCols];
+        tmem_ld_32x32b_x32(my_s, sv);
         tmem_ld_wait();
 #pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          unpack_f32x2(fma_f32x2(pack_u32x2(sv[2 * e], sv[2 * e + 1]), sc2, DQ ? own_nlse : rv[e]), pe[2 * e], pe[2 * e + 1]);
+        for (int e = 0; e < kBwdCols / 2; ++e) {
+          unpack_f32x2(fma_f32x2(pack_u32x2(sv[2 * e], sv[2 * e + 1]), sc2, DQ ? own_nlse : nlse[e]), pe[2 * e], pe[2 * e + 1]);
           pe[2 * e] = exp2f(pe[2 * e]);
           pe[2 * e + 1] = exp2f(pe[2 * e + 1]);
         }
       }
-      if (need_mask) mask_row(pe, c0 + half * 64);
+      if (need_mask) mask_row(pe, c0 + part * kBwdCols);
       if (!DQ) {
-        uint32_t pk[32];
+        uint32_t pk[kBwdCols / 2];
 #pragma unroll
-        for (int e = 0; e < 32; ++e) pk[e] = pack_bf16x2(pe[2 * e], pe[2 * e + 1]);
-        tmem_st_32x32b_x32(my_s, pk);
+        for (int e = 0; e < kBwdCols / 2; ++e) pk[e] = pack_bf16x2(pe[2 * e], pe[2 * e + 1]);
+        tmem_st_32x32b_x16(my_s, pk);
         tmem_st_wait();
       }
+      // dO_i has to be there for dV now; its buffer, and with it this barrier's phase, may be reused from here on
+      if (!DQ && !__all_sync(0xffffffffu, mbar_wait(full_bar(2 * i + 1), full_phase(2 * i + 1), p.status, abort_flag))) { ok = false; break; }
       tc_fence_before();
       mbar_arrive(smem_u32(p_ready));
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(dp_full), i & 1, p.status, abort_flag))) { ok = false; break; }
       tc_fence_after();
       {
-        uint32_t dv[64], pk[32];
-        tmem_ld_32x32b_x32(my_dp, *reinterpret_cast<uint32_t(*)[32]>(dv));
-        tmem_ld_32x32b_x32(my_dp + 32, *reinterpret_cast<uint32_t(*)[32]>(dv + 32));
+        uint32_t dv[kBwdCols], pk[kBwdCols / 2];
+        tmem_ld_32x32b_x32(my_dp, dv);
         tmem_ld_wait();
 #pragma unroll
-        for (int e = 0; e < 32; ++e)
+        for (int e = 0; e < kBwdCols / 2; ++e)
           unpack_f32x2(mul_f32x2(pack_f32x2(pe[2 * e], pe[2 * e + 1]),
-                                 add_f32x2(pack_u32x2(dv[2 * e], dv[2 * e + 1]), DQ ? own_ndelta : rv[64 + e])),
+                                 add_f32x2(pack_u32x2(dv[2 * e], dv[2 * e + 1]), DQ ? own_ndelta : ndelta[e])),
                        pe[2 * e], pe[2 * e + 1]);
-        if (need_mask) mask_row(pe, c0 + half * 64);         // 0 * inf from elements that do not count
+        if (need_mask) mask_row(pe, c0 + part * kBwdCols);         // 0 * inf from elements that do not count
 #pragma unroll
-        for (int e = 0; e < 32; ++e) pk[e] = pack_bf16x2(pe[2 * e], pe[2 * e + 1]);
-        tmem_st_32x32b_x32(my_dp, pk);
+        for (int e = 0; e < kBwdCols / 2; ++e) pk[e] = pack_bf16x2(pe[2 * e], pe[2 * e + 1]);
+        tmem_st_32x32b_x16(my_dp, pk);
         tmem_st_wait();
       }
       tc_fence_before();
@@ -783,24 +813,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_consta
 #pragma unroll
       for (int a = (DQ ? 1 : 0); a < 2; ++a) {
         // acc0 = dV (columns 2H..); acc1 = dK (columns H..) or dQ (columns 0..), whose factor is applied here, once,
-        // to the fp32 sums; each half stores 64 columns
-        __nv_bfloat16* dst = grow + (DQ ? 0 : (a == 0 ? 2 * H : H)) + half * 64;
+        // to the fp32 sums; each thread stores 32 columns
+        __nv_bfloat16* dst = grow + (DQ ? 0 : (a == 0 ? 2 * H : H)) + part * kBwdCols;
         const float f = a == 0 ? 1.f : p.scale;
+        uint32_t t4[kBwdCols];
+        tmem_ld_32x32b_x32((a == 0 ? tmem_acc0 : tmem_acc1) + lane_off + part * kBwdCols, t4);
+        tmem_ld_wait();
+        if (!row_ok) continue;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t t4[32];
-          tmem_ld_32x32b_x32((a == 0 ? tmem_acc0 : tmem_acc1) + lane_off + half * 64 + c * 32, t4);
-          tmem_ld_wait();
-          if (!row_ok) continue;
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint4 o;
-            o.x = pack_bf16x2(__uint_as_float(t4[g * 8 + 0]) * f, __uint_as_float(t4[g * 8 + 1]) * f);
-            o.y = pack_bf16x2(__uint_as_float(t4[g * 8 + 2]) * f, __uint_as_float(t4[g * 8 + 3]) * f);
-            o.z = pack_bf16x2(__uint_as_float(t4[g * 8 + 4]) * f, __uint_as_float(t4[g * 8 + 5]) * f);
-            o.w = pack_bf16x2(__uint_as_float(t4[g * 8 + 6]) * f, __uint_as_float(t4[g * 8 + 7]) * f);
-            *reinterpret_cast<uint4*>(dst + c * 32 + g * 8) = o;
-          }
+        for (int g = 0; g < kBwdCols / 8; ++g) {
+          uint4 o;
+          o.x = pack_bf16x2(__uint_as_float(t4[g * 8 + 0]) * f, __uint_as_float(t4[g * 8 + 1]) * f);
+          o.y = pack_bf16x2(__uint_as_float(t4[g * 8 + 2]) * f, __uint_as_float(t4[g * 8 + 3]) * f);
+          o.z = pack_bf16x2(__uint_as_float(t4[g * 8 + 4]) * f, __uint_as_float(t4[g * 8 + 5]) * f);
+          o.w = pack_bf16x2(__uint_as_float(t4[g * 8 + 6]) * f, __uint_as_float(t4[g * 8 + 7]) * f);
+          *reinterpret_cast<uint4*>(dst + g * 8) = o;
         }
       }
     }
