@@ -230,7 +230,9 @@ class _FusedCEFn(torch.autograd.Function):
     def backward(ctx, dloss):
         (dlogits,) = ctx.saved_tensors
         if not ctx.unit_upstream_grad:
-            dlogits.mul_(dloss.to(dlogits.dtype))
+            from . import kernels as K
+
+            K.scale_bf16_(dlogits, dloss.float())
         return dlogits, None, None, None, None
 
 

@@ -282,8 +282,8 @@ def embedding_bwd(dy: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, accumu
     assert out.shape[1] == H and ids.numel() == T
     key = (V, T, str(dy.device))
     work = _EMBED_WORK.get(key)
-    if work is None:      # count | start | order; reused by every call of this size (calls are stream-ordered)
-        work = _EMBED_WORK[key] = torch.empty(2 * V + T, dtype=torch.int32, device=dy.device)
+    if work is None:      # count | cursor | place | order; reused by every call of this size (calls are stream-ordered)
+        work = _EMBED_WORK[key] = torch.empty(2 * V + 2 * T, dtype=torch.int32, device=dy.device)
     _lib.check(_L().mfsdp_embedding_bwd(dy.data_ptr(), dy.stride(0), ids.data_ptr(), out.data_ptr(), out.stride(0),
                                         T, V, H, int(accumulate), work.data_ptr(), _stream()), "embedding_bwd")
     return out
@@ -413,3 +413,11 @@ def cast_bf16_f32(src: torch.Tensor, dst: torch.Tensor) -> None:
     assert src.dtype == torch.bfloat16 and dst.dtype == torch.float32 and src.numel() == dst.numel()
     assert src.is_contiguous() and dst.is_contiguous()
     _lib.check(_L().mfsdp_cast_bf16_f32(src.data_ptr(), dst.data_ptr(), src.numel(), _stream()), "cast_bf16_f32")
+
+
+def scale_bf16_(x: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:
+    """``x *= scale`` for a contiguous bf16 tensor and a one-element fp32 device tensor (no host read)."""
+    assert x.dtype == torch.bfloat16 and x.is_contiguous()
+    assert scale.dtype == torch.float32 and scale.numel() == 1 and scale.device == x.device
+    _lib.check(_L().mfsdp_scale_bf16(x.data_ptr(), x.numel(), scale.data_ptr(), _stream()), "scale_bf16")
+    return x

@@ -44,6 +44,7 @@ _SIGNATURES: dict[str, list] = {
     "mfsdp_muon_apply_many": [vp, vp, i32, vp, i64, f32, f32, f32, vp],
     "mfsdp_copy_segments": [vp, vp, vp, vp, vp, i32, i64, i32, vp],
     "mfsdp_cast_f32_bf16": [vp, vp, i64, vp],
+    "mfsdp_scale_bf16": [vp, i64, vp, vp],
     "mfsdp_cast_bf16_f32": [vp, vp, i64, vp],
 }
 

@@ -437,3 +437,28 @@ def test_adamw_of_parameters_outside_units(n, with_lp, aligned):
         assert (id(p) in opt.lp_written) == (with_lp and aligned)
         if with_lp and aligned:
             assert torch.equal(lp, p.detach().bfloat16())
+
+
+@pytest.mark.parametrize("T,V,H,ids", [(1, 8, 8, "one"), (300, 5000, 264, "all the same"), (3000, 4097, 72, "few"), (4096, 4096, 2056, "uniform")])
+def test_embedding_backward_orders_positions(K, T, V, H, ids):
+    """Ids that occur once, up to and beyond the 256 positions that a block sorts, and not at all: the same bits every
+    time, within one bf16 rounding of the 64-bit sums plus fp32 rounding of n terms."""
+    g = torch.Generator(device="cuda").manual_seed(T)
+    t = dict(zip(("one", "all the same", "few", "uniform"),
+                 (lambda: torch.full((T,), V - 1), lambda: torch.full((T,), 7), lambda: torch.randint(0, 9, (T,)) * 455,
+                  lambda: torch.randint(0, V, (T,)))))[ids]().to("cuda", torch.int64)
+    dy = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    outs = [K.embedding_bwd(dy, t, torch.full((V, H), float("nan"), device="cuda", dtype=torch.bfloat16)) for _ in range(3)]
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    want = torch.zeros(V, H, dtype=torch.float64, device="cuda").index_add_(0, t, dy.double())
+    size = torch.zeros(V, H, dtype=torch.float64, device="cuda").index_add_(0, t, dy.double().abs())
+    assert ((outs[0].double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -23 * T * size).all()
+
+
+@pytest.mark.parametrize("n,shift,f", [(1, 0, 0.5), (7, 0, -3.0), (4103, 0, 0.3), (4096, 1, 0.3), (4096, 0, 1.0)])
+def test_scale_bf16(K, n, shift, f):
+    """One fp32 product and one rounding per element: exact against the same in torch."""
+    x = torch.randn(n + shift, device="cuda").bfloat16()[shift:]
+    s = torch.tensor(f, device="cuda")
+    want = (x.float() * s).bfloat16()
+    assert torch.equal(K.scale_bf16_(x, s), want)
