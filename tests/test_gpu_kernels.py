@@ -462,3 +462,49 @@ def test_scale_bf16(K, n, shift, f):
     s = torch.tensor(f, device="cuda")
     want = (x.float() * s).bfloat16()
     assert torch.equal(K.scale_bf16_(x, s), want)
+
+
+@pytest.mark.parametrize("rows,V,pad", [(1, 8, 0), (5, 1016, 8), (700, 1032, 0), (149, 4104, 0), (450, 16392, 0), (300, 32760, 8), (297, 49152, 0)])
+def test_cross_entropy_block_sizes(K, rows, V, pad):
+    """Every block size, vectors that do not divide the block, row pitches above V; ignored targets, -inf logits in
+    whole threads' shares.  Loss: fp32 sums (1e-5); gradient: one bf16 rounding."""
+    torch.manual_seed(rows)
+    logits = (3 * torch.randn(rows, V + pad, device="cuda")).bfloat16()
+    logits[:, V // 2:] -= 2.0
+    if V > 64:
+        logits[rows // 2, 8:V - 8] = -math.inf
+    target = torch.randint(0, V, (rows,), device="cuda")
+    target[rows // 2] = 0
+    if rows > 2:
+        target[1] = -100
+    x = logits[:, :V].double().requires_grad_(True)
+    want = torch.nn.functional.cross_entropy(x, target, ignore_index=-100, reduction="none")
+    (grad,) = torch.autograd.grad(want.sum() * 0.25, x)
+    tail = logits[:, V:].clone()
+    loss = K.cross_entropy_(logits[:, :V], target, 0.25)
+    K.check_status()
+    assert (loss.double() - want).abs().max() <= 1e-5 * max(1.0, want.abs().max().item())
+    assert ((logits[:, :V].double() - grad).abs() <= 2 ** -8 * grad.abs() + 1e-7).all()
+    assert torch.equal(logits[:, V:], tail)
+
+
+@pytest.mark.parametrize("rows", [1, 7, 9, 1185, 2500])
+@pytest.mark.parametrize("H", [8, 264, 520, 1032, 2056, 4104, 8192])
+def test_rmsnorm_rows_and_widths(K, rows, H):
+    """One, two and four warps per row with remainders, fewer rows than a block takes, one and several trips.  Bounds: one
+    bf16 rounding per element (2^-8) of values whose fp32 terms are a few rounding errors off."""
+    torch.manual_seed(rows + H)
+    x, w = _rand(rows, H), (1 + 0.1 * torch.randn(H, device="cuda")).bfloat16()
+    dy, dres = _rand(rows, H), _rand(rows, H)
+    y, rstd = K.rmsnorm_fwd(x, w, 1e-5)
+    xd, wd = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    ref = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-5) * wd
+    ref.backward(dy.double())
+    assert _rel_err(y, ref) < 2 ** -8 and torch.allclose(rstd.double(), torch.rsqrt(x.double().pow(2).mean(-1) + 1e-5), rtol=1e-5)
+    for res in (dres, None):
+        old = torch.randn(H, device="cuda").bfloat16()
+        acc = old.clone()
+        dx, dw = K.rmsnorm_bwd(dy, x, w, rstd, dres=res, dw_out=acc, accumulate_dw=res is None)
+        assert _rel_err(dx, xd.grad + (res.double() if res is not None else 0)) < 2 ** -7
+        assert _rel_err(acc, wd.grad + (old.double() if res is None else 0)) < 2 ** -7
+        assert dw is acc
