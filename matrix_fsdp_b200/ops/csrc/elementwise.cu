@@ -768,11 +768,11 @@ static inline int grid_for(long long work, int threads, int max_blocks = 148 * 8
 
 // ============================================================== embedding backward
 // dW[v, :] = sum over the positions t with ids[t] == v of dy[t, :], written (or accumulated) straight into
-// the gradient bucket.  Count per id, exclusive scan over the vocabulary, positions dropped into their id's range in
+// the gradient bucket.  Count per id, a range of a list for every id, positions dropped into their id's range in
 // whatever order the atomics take; then one CTA per vocabulary row puts its few positions into ascending order and
 // sums them, so the fp32 sum of a row is the same in every run, and writes the row once, zeros where an id does not
 // occur: no separate fill of the V x H gradient, no atomics on values.  (Ranking every position among all earlier ones
-// took 290 us for 16384 positions, the scan with strided reads 55 us for 32000 ids.)
+// took 290 us for 16384 positions, ranges in the order of the ids by one block's scan 28 us for 32000 ids.)
 __global__ void embed_count_kernel(const long long* __restrict__ ids, int T, int V, int* __restrict__ count) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T) return;
@@ -780,42 +780,32 @@ __global__ void embed_count_kernel(const long long* __restrict__ ids, int T, int
   if (v >= 0 && v < V) atomicAdd(&count[v], 1);
 }
 
-__global__ void __launch_bounds__(1024) embed_scan_kernel(const int* __restrict__ count, int* __restrict__ cursor, int V) {
-  __shared__ int warp_sum_of[32];
+// Gives every id a range of `place` as long as its count; which range does not matter, so a block's ids are numbered
+// among themselves and one atomic takes their part of the whole.
+__global__ void __launch_bounds__(256) embed_range_kernel(const int* __restrict__ count, int* __restrict__ cursor, int V,
+                                                          int* __restrict__ taken) {
+  __shared__ int warp_total[8];
+  __shared__ int block_start;
+  const int v = blockIdx.x * 256 + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int run = 0;                                        // ids below `base`
-  for (int base = 0; base < V; base += 4096) {
-    const int i = base + threadIdx.x * 4;
-    int c[4], s = 0;
+  const int c = v < V ? count[v] : 0;
+  int incl = c;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      c[k] = i + k < V ? count[i + k] : 0;
-      s += c[k];
-    }
-    int incl = s;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += o;
-    }
-    __syncthreads();                                  // the previous round's sums have been read
-    if (lane == 31) warp_sum_of[warp] = incl;
-    __syncthreads();
-    int w = warp_sum_of[lane];                        // every warp scans the 32 sums for itself
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, w, off);
-      if (lane >= off) w += o;
-    }
-    const int before = __shfl_sync(0xffffffffu, w, warp) - __shfl_sync(0xffffffffu, incl, 31);
-    int pos = run + before + incl - s;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (i + k < V) cursor[i + k] = pos;
-      pos += c[k];
-    }
-    run += __shfl_sync(0xffffffffu, w, 31);
+  for (int off = 1; off < 32; off <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += o;
   }
+  if (lane == 31) warp_total[warp] = incl;
+  __syncthreads();
+  int before = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    if (w < warp) before += warp_total[w];
+    total += warp_total[w];
+  }
+  if (threadIdx.x == 0) block_start = total > 0 ? atomicAdd(taken, total) : 0;
+  __syncthreads();
+  if (v < V) cursor[v] = block_start + before + incl - c;
 }
 
 // Afterwards cursor[v] is the end of v's range.
@@ -981,20 +971,21 @@ MFSDP_API int mfsdp_swiglu_fwd(const void* gu, void* h, long long T, int F, cuda
   return (int)cudaGetLastError();
 }
 
-// dW[V, H] (row pitch lddw) from dy[T, H] (row pitch lddy) and ids[T]; `work` holds 2 * V + 2 * T ints.  Ids outside
+// dW[V, H] (row pitch lddw) from dy[T, H] (row pitch lddy) and ids[T]; `work` holds 2 * V + 2 * T + 1 ints.  Ids outside
 // [0, V) contribute nothing.  accumulate != 0 adds to what dW holds (rows whose id does not occur stay as they are).
 MFSDP_API int mfsdp_embedding_bwd(const void* dy, long long lddy, const long long* ids, void* dw, long long lddw,
                                   int T, int V, int H, int accumulate, int* work, cudaStream_t st) {
   if (T <= 0 || V <= 0 || H <= 0 || (H % 8) || (lddy % 8) || (lddw % 8)) return -2;
   if (((uintptr_t)dy & 15) || ((uintptr_t)dw & 15)) return -2;
   int* count = work;
-  int* cursor = work + V;
-  int* place = work + 2 * (long long)V;
+  int* taken = work + V;
+  int* cursor = taken + 1;
+  int* place = cursor + V;
   int* order = place + T;
-  cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int) * (size_t)V, st);
+  cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int) * ((size_t)V + 1), st);
   if (e != cudaSuccess) return (int)e;
   embed_count_kernel<<<(T + 255) / 256, 256, 0, st>>>(ids, T, V, count);
-  embed_scan_kernel<<<1, 1024, 0, st>>>(count, cursor, V);
+  embed_range_kernel<<<(V + 255) / 256, 256, 0, st>>>(count, cursor, V, taken);
   embed_place_kernel<<<(T + 255) / 256, 256, 0, st>>>(ids, T, V, cursor, place);
   embed_sum_kernel<<<V, 256, 0, st>>>((const __nv_bfloat16*)dy, lddy, (__nv_bfloat16*)dw, lddw, H, ids, T, count, cursor,
                                       place, order, accumulate);

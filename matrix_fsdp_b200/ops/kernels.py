@@ -282,8 +282,8 @@ def embedding_bwd(dy: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, accumu
     assert out.shape[1] == H and ids.numel() == T
     key = (V, T, str(dy.device))
     work = _EMBED_WORK.get(key)
-    if work is None:      # count | cursor | place | order; reused by every call of this size (calls are stream-ordered)
-        work = _EMBED_WORK[key] = torch.empty(2 * V + 2 * T, dtype=torch.int32, device=dy.device)
+    if work is None:      # count | taken | cursor | place | order; reused by every call of this size (calls are stream-ordered)
+        work = _EMBED_WORK[key] = torch.empty(2 * V + 2 * T + 1, dtype=torch.int32, device=dy.device)
     _lib.check(_L().mfsdp_embedding_bwd(dy.data_ptr(), dy.stride(0), ids.data_ptr(), out.data_ptr(), out.stride(0),
                                         T, V, H, int(accumulate), work.data_ptr(), _stream()), "embedding_bwd")
     return out
