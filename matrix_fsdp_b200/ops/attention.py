@@ -78,7 +78,7 @@ def attention_fwd(qkv: torch.Tensor, batch: int, seq: int, n_heads: int, head_di
     lib = _lib.load()
     _lib.check(lib.mfsdp_attention_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), batch, seq, n_heads,
                                        qkv.stride(0), out.stride(0), scale, status.data_ptr(),
-                                       torch.cuda.current_stream(qkv.device).cuda_stream),
+                                       torch._C._cuda_getCurrentRawStream(qkv.get_device())),
                "mfsdp_attention_fwd")
     return out, lse
 
@@ -103,6 +103,6 @@ def attention_bwd(dout: torch.Tensor, qkv: torch.Tensor, out: torch.Tensor, lse:
     _lib.check(lib.mfsdp_attention_bwd(dout.data_ptr(), qkv.data_ptr(), out.data_ptr(), lse.data_ptr(),
                                        dqkv.data_ptr(), scratch.data_ptr(), batch, seq, n_heads, qkv.stride(0), dout.stride(0),
                                        dqkv.stride(0), scale, status.data_ptr(),
-                                       torch.cuda.current_stream(qkv.device).cuda_stream),
+                                       torch._C._cuda_getCurrentRawStream(qkv.get_device())),
                "mfsdp_attention_bwd")
     return dqkv

@@ -20,6 +20,7 @@ from . import lib as _lib
 
 _STATUS: dict[int, torch.Tensor] = {}
 _SM_COUNT: dict[int, int] = {}
+_CONTEXT: dict[torch.device, tuple[int, int]] = {}
 _SCRATCH: dict[tuple, torch.Tensor] = {}
 
 
@@ -32,7 +33,19 @@ def launch_count() -> int:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Raw handle of the current stream.  (``torch.cuda.current_stream()`` builds a stream object behind five Python
+    frames on every launch: a fifth of the host time of a step whose kernels are short.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def _launch_context(device: torch.device) -> tuple[int, int]:
+    """Address of the device's status word and its number of SMs."""
+    ctx = _CONTEXT.get(device)
+    if ctx is None:
+        ctx = (status_word(device).data_ptr(), sm_count(device))
+        if device.index is not None:           # "cuda" without an index names whichever device is current
+            _CONTEXT[device] = ctx
+    return ctx
 
 
 def status_word(device: torch.device | int | None = None) -> torch.Tensor:
@@ -111,7 +124,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
         a.data_ptr(), b.data_ptr(), out.data_ptr(), cin.data_ptr() if cin is not None else None,
         M, N, K, a.stride(0), b.stride(0), out.stride(0), cin.stride(0) if cin is not None else 0,
         int(a_mn_major), int(b_mn_major), float(alpha), float(beta), 0, None, None, 0, 0,
-        status_word(a.device).data_ptr(), sm_count(a.device), force_bn, _stream())
+        *_launch_context(a.device), force_bn, _stream())
     _lib.check(rc, "mfsdp_gemm_bf16")
     return out
 
@@ -137,7 +150,7 @@ def gemm_ag(a: torch.Tensor, b: torch.Tensor, plan, *, out: torch.Tensor | None 
         plan.src.data_ptr(), plan.dst.data_ptr(), plan.nbytes.data_ptr(), plan.flag_idx.data_ptr(), plan.njobs,
         plan.flags.data_ptr(), plan.need.data_ptr(), plan.first.data_ptr(), int(plan.rotate), plan.bn,
         int(plan.budget_ns),
-        status_word(a.device).data_ptr(), sm_count(a.device), _stream())
+        *_launch_context(a.device), _stream())
     _lib.check(rc, "mfsdp_gemm_bf16_ag")
     return out
 
@@ -178,7 +191,7 @@ def grouped_gemm_m(a: torch.Tensor, b: torch.Tensor, tile_group: torch.Tensor, *
         a.data_ptr(), b.data_ptr(), out.data_ptr(), cin.data_ptr() if cin is not None else None, Mtot, N, K,
         a.stride(0), ldb, out.stride(0), cin.stride(0) if cin is not None else 0, 0, int(b_mn_major),
         float(alpha), float(beta), 1, tile_group.data_ptr(), None, G, 0,
-        status_word(a.device).data_ptr(), sm_count(a.device), 2 if groups_of_256_rows and Mtot % 256 == 0 else 0, _stream())
+        *_launch_context(a.device), 2 if groups_of_256_rows and Mtot % 256 == 0 else 0, _stream())
     _lib.check(rc, "mfsdp_gemm_bf16[m-grouped]")
     return out
 
@@ -201,7 +214,7 @@ def grouped_gemm_k(a: torch.Tensor, b: torch.Tensor, group_offsets: torch.Tensor
     rc = (_L().mfsdp_gemm_bf16_sym if symmetric else _L().mfsdp_gemm_bf16)(
         a.data_ptr(), b.data_ptr(), out.data_ptr(), None, M, N, 0, a.stride(0), b.stride(0), N, 0,
         1, 1, 1.0, 0.0, 2, None, group_offsets.data_ptr(), num_groups, Ktot,
-        status_word(a.device).data_ptr(), sm_count(a.device), 0, _stream())
+        *_launch_context(a.device), 0, _stream())
     _lib.check(rc, "mfsdp_gemm_bf16[k-grouped]")
     return out
 

@@ -11,6 +11,7 @@ import ctypes as C
 import torch
 
 from . import lib as _lib
+from .kernels import _stream as _st
 
 _vp, _i, _ll, _f = C.c_void_p, C.c_int, C.c_longlong, C.c_float
 
@@ -33,8 +34,6 @@ def _L():
     return _lib.load(required=True)
 
 
-def _st() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 def _p(t: torch.Tensor | None):
