@@ -536,7 +536,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs 
 
 
 // =============================================================================== backward
-// Two kernels without atomics (the sums have one order in every run), sharing one body:
+// Two kinds of block without atomics (the sums have one order in every run), sharing one body:
 //   DQ = false: one CTA per (batch, head, 128-key tile).  K_j and V_j stay in shared memory, the query axis streams
 //               in tiles of 128 rows (Q_i, dO_i).  S^T = K_j Q_i^T and dP^T = V_j dO_i^T land in TMEM (thread = key
 //               row, four threads per row), P^T and dS^T go back over them as bf16, dV += P^T dO_i and dK += dS^T Q_i
@@ -597,9 +597,8 @@ __device__ __forceinline__ void mma_acc_ts(uint32_t tmem_d, uint32_t tmem_p, uin
 }
 
 template <bool DQ>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_constant__ CUtensorMap tma_do,
-                const AttnBwdArgs p) {
+__device__ __forceinline__ void attn_bwd_block(const CUtensorMap& tma_qkv, const CUtensorMap& tma_do, const AttnBwdArgs& p,
+                                               const int block) {
   extern __shared__ __align__(1024) uint8_t smem[];
   if (smem_u32(smem) & 1023) {         // the swizzled tiles need it; nothing has been started yet
     if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, (int)kErrBadArgument);
@@ -620,8 +619,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Blocks in the order of attn_fwd2_kernel: per group of heads the long tiles first.
   const int nt = (p.S + 127) / 128, nheads = p.nH * p.B;
-  const int grp = (int)blockIdx.x / (p.heads_per_group * nt);
-  const int in_grp = (int)blockIdx.x - grp * p.heads_per_group * nt;
+  const int grp = block / (p.heads_per_group * nt);
+  const int in_grp = block - grp * p.heads_per_group * nt;
   const int gheads = min(p.heads_per_group, nheads - grp * p.heads_per_group);
   const int nth = in_grp / gheads;
   const int bh = grp * p.heads_per_group + in_grp % gheads;
@@ -841,6 +840,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_consta
   }
 }
 
+// Both kinds of block in one grid, dK / dV first, so that the first kind's last wave is filled by the long blocks of the
+// second (a head of 1024 rows has 8 blocks of each kind, 1 to 8 tiles long).  Two launches -> one, preparation included:
+// 16 heads of 1024 rows 51.5 -> 36.6 us, of 4 x 1024 132 -> 120 us, of 3 x 1333 155 -> 143 us, 8 heads of 8192 rows 478 ->
+// 441 us.  Alternating kinds were slower at long rows, where each streams tensors of its own through the L2.
+__global__ void __launch_bounds__(kBwdThreads, 1)
+attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_constant__ CUtensorMap tma_do,
+                const __grid_constant__ AttnBwdArgs p) {
+  const int n = (int)(gridDim.x >> 1), block = (int)blockIdx.x;
+  if (block < n) attn_bwd_block<false>(tma_qkv, tma_do, p, block);
+  else attn_bwd_block<true>(tma_qkv, tma_do, p, block - n);
+}
+
 // nlse2 = -lse * log2(e); ndelta = -rowsum(dO * O); both zero for the rows that pad a head to whole tiles.  Half a
 // warp per (row, head), 16 bytes of each operand per lane.
 __global__ void __launch_bounds__(256)
@@ -935,9 +946,7 @@ MFSDP_API int mfsdp_attention_bwd(const void* dout, const void* qkv, const void*
   if (rc) return rc;
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnBwdSmem::kBytes);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attn_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnBwdSmem::kBytes);
+    cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnBwdSmem::kBytes);
     if (e != cudaSuccess) return (int)e;
     attr = true;
   }
@@ -953,8 +962,6 @@ MFSDP_API int mfsdp_attention_bwd(const void* dout, const void* qkv, const void*
   a.nlse2 = nlse2; a.ndelta = ndelta;
   a.dqkv = (__nv_bfloat16*)dqkv; a.ld_dqkv = ld_dqkv; a.status = status;
   a.heads_per_group = heads_in_l2(B, S, nH);
-  const unsigned grid = (unsigned)(nt * B * nH);
-  attn_bwd_kernel<false><<<grid, kBwdThreads, AttnBwdSmem::kBytes, st>>>(map_qkv, map_do, a);
-  attn_bwd_kernel<true><<<grid, kBwdThreads, AttnBwdSmem::kBytes, st>>>(map_qkv, map_do, a);
+  attn_bwd_kernel<<<2u * (unsigned)(nt * B * nH), kBwdThreads, AttnBwdSmem::kBytes, st>>>(map_qkv, map_do, a);
   return (int)cudaGetLastError();
 }
