@@ -883,9 +883,16 @@ __global__ void __launch_bounds__(256) embed_sum_kernel(const __nv_bfloat16* __r
   }
 }
 
+__device__ __forceinline__ void put8(float* p, const float (&f)[8]) { store8(p, f); }
+__device__ __forceinline__ void put8(__nv_bfloat16* p, const float (&f)[8]) { *reinterpret_cast<uint4*>(p) = pack8(f); }
+__device__ __forceinline__ void put1(float* p, float v) { *p = v; }
+__device__ __forceinline__ void put1(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
+
 // x *= *scale in fp32, 8 elements per access; nothing to do for a scale of one (a loss that is what backward() is called
-// on).  The library's bf16 product with a one-element tensor moved 262 M logits in 677 us, 1.5 TB/s.
-__global__ void __launch_bounds__(256) scale_bf16_kernel(__nv_bfloat16* __restrict__ x, long long n, const float* __restrict__ scale) {
+// on, a gradient below the clipping threshold).  The library's bf16 product with a one-element tensor moved 262 M logits
+// in 677 us, 1.5 TB/s.
+template <typename T>
+__global__ void __launch_bounds__(256) scale_kernel(T* __restrict__ x, long long n, const float* __restrict__ scale) {
   const float f = *scale;
   if (f == 1.f) return;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -897,9 +904,30 @@ __global__ void __launch_bounds__(256) scale_bf16_kernel(__nv_bfloat16* __restri
     load8(x + i * 8, v);
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] *= f;
-    reinterpret_cast<uint4*>(x)[i] = pack8(v);
+    put8(x + i * 8, v);
   }
-  for (long long i = nv * 8 + tid; i < n; i += stride) x[i] = __float2bfloat16_rn(__bfloat162float(x[i]) * f);
+  for (long long i = nv * 8 + tid; i < n; i += stride) put1(x + i, to_float(x[i]) * f);
+}
+
+// partial[block] = sum of squares of the block's share, in fp32; reads bf16 as it is (a widened copy of every gradient
+// shard and its norm took 71 us for 34 M elements).
+template <typename T>
+__global__ void __launch_bounds__(256) sumsq_kernel(const T* __restrict__ x, long long n, float* __restrict__ partial) {
+  __shared__ float red[32];
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long nv = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? n >> 3 : 0;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (long long i = tid; i < nv; i += stride) {
+    float v[8];
+    load8(x + i * 8, v);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e & 3] += v[e] * v[e];
+  }
+  for (long long i = nv * 8 + tid; i < n; i += stride) acc[0] += to_float(x[i]) * to_float(x[i]);
+  const float sum = block_sum((acc[0] + acc[1]) + (acc[2] + acc[3]), red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = sum;
 }
 
 }  // namespace mfsdp
@@ -1171,9 +1199,20 @@ MFSDP_API int mfsdp_cast_f32_bf16(const float* src, void* dst, long long n, cuda
   return (int)cudaGetLastError();
 }
 
-MFSDP_API int mfsdp_scale_bf16(void* x, long long n, const float* scale, cudaStream_t st) {
+MFSDP_API int mfsdp_scale(void* x, int is_bf16, long long n, const float* scale, cudaStream_t st) {
   if (n <= 0) return 0;
-  scale_bf16_kernel<<<grid_for(n / 8 + 1, 256, 148 * 8), 256, 0, st>>>((__nv_bfloat16*)x, n, scale);
+  const int grid = grid_for(n / 8 + 1, 256, 148 * 8);
+  if (is_bf16) scale_kernel<<<grid, 256, 0, st>>>((__nv_bfloat16*)x, n, scale);
+  else scale_kernel<<<grid, 256, 0, st>>>((float*)x, n, scale);
+  return (int)cudaGetLastError();
+}
+
+// `partial`: kSumsqBlocks floats, all of them written.
+constexpr int kSumsqBlocks = 148 * 4;
+MFSDP_API int mfsdp_sumsq(const void* x, int is_bf16, long long n, float* partial, cudaStream_t st) {
+  if (n < 0) return -2;
+  if (is_bf16) sumsq_kernel<<<kSumsqBlocks, 256, 0, st>>>((const __nv_bfloat16*)x, n, partial);
+  else sumsq_kernel<<<kSumsqBlocks, 256, 0, st>>>((const float*)x, n, partial);
   return (int)cudaGetLastError();
 }
 

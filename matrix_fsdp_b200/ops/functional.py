@@ -232,7 +232,7 @@ class _FusedCEFn(torch.autograd.Function):
         if not ctx.unit_upstream_grad:
             from . import kernels as K
 
-            K.scale_bf16_(dlogits, dloss.float())
+            K.scale_(dlogits, dloss.float())
         return dlogits, None, None, None, None
 
 

@@ -428,9 +428,17 @@ def cast_bf16_f32(src: torch.Tensor, dst: torch.Tensor) -> None:
     _lib.check(_L().mfsdp_cast_bf16_f32(src.data_ptr(), dst.data_ptr(), src.numel(), _stream()), "cast_bf16_f32")
 
 
-def scale_bf16_(x: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:
-    """``x *= scale`` for a contiguous bf16 tensor and a one-element fp32 device tensor (no host read)."""
-    assert x.dtype == torch.bfloat16 and x.is_contiguous()
+def scale_(x: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:
+    """``x *= scale`` for a contiguous bf16 or fp32 tensor and a one-element fp32 device tensor (no host read)."""
+    assert x.dtype in (torch.bfloat16, torch.float32) and x.is_contiguous()
     assert scale.dtype == torch.float32 and scale.numel() == 1 and scale.device == x.device
-    _lib.check(_L().mfsdp_scale_bf16(x.data_ptr(), x.numel(), scale.data_ptr(), _stream()), "scale_bf16")
+    _lib.check(_L().mfsdp_scale(x.data_ptr(), int(x.dtype == torch.bfloat16), x.numel(), scale.data_ptr(), _stream()), "scale")
     return x
+
+
+def sumsq(x: torch.Tensor) -> torch.Tensor:
+    """Sum of squares of a contiguous bf16 or fp32 tensor, a 0-dim fp32 tensor."""
+    assert x.dtype in (torch.bfloat16, torch.float32) and x.is_contiguous()
+    partial = torch.empty(148 * 4, dtype=torch.float32, device=x.device)
+    _lib.check(_L().mfsdp_sumsq(x.data_ptr(), int(x.dtype == torch.bfloat16), x.numel(), partial.data_ptr(), _stream()), "sumsq")
+    return partial.sum()

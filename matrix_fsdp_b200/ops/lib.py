@@ -44,7 +44,8 @@ _SIGNATURES: dict[str, list] = {
     "mfsdp_muon_apply_many": [vp, vp, i32, vp, i64, f32, f32, f32, vp],
     "mfsdp_copy_segments": [vp, vp, vp, vp, vp, i32, i64, i32, vp],
     "mfsdp_cast_f32_bf16": [vp, vp, i64, vp],
-    "mfsdp_scale_bf16": [vp, i64, vp, vp],
+    "mfsdp_scale": [vp, i32, i64, vp, vp],
+    "mfsdp_sumsq": [vp, i32, i64, vp, vp],
     "mfsdp_cast_bf16_f32": [vp, vp, i64, vp],
 }
 
@@ -97,7 +98,7 @@ def available() -> bool:
 
 
 # kernels launched per launcher call (default 1); the counter feeds the benchmark's launch report
-_KERNELS_PER_CALL = {"rmsnorm_bwd": 2, "muon_prepare_many": 2, "mfsdp_attention_bwd": 3}
+_KERNELS_PER_CALL = {"rmsnorm_bwd": 2, "muon_prepare_many": 2, "mfsdp_attention_bwd": 2}
 _LAUNCH_COUNT = [0]
 
 

@@ -74,6 +74,21 @@ def clip_grad_norm_(module_or_units, max_norm: float, norm_type: float = 2.0,
 
     units = collect_param_groups(module_or_units)
     inf = math.isinf(norm_type)
+
+    def kernels_for(g):
+        if not g.is_cuda or not g.is_contiguous() or g.dtype not in (torch.bfloat16, torch.float32):
+            return None
+        from ..ops import kernels, lib
+
+        return kernels if lib.available() and not lib.disabled_by_env() else None
+
+    def power_sum(g):
+        g = g.detach()
+        if inf:
+            return g.float().abs().max()
+        K = kernels_for(g) if norm_type == 2.0 else None
+        return K.sumsq(g) if K is not None else g.float().norm(norm_type).pow(norm_type)
+
     per_group: dict[object, tuple[object, torch.Tensor]] = {}
     shards = []
     for u in units:
@@ -82,7 +97,7 @@ def clip_grad_norm_(module_or_units, max_norm: float, norm_type: float = 2.0,
         if g is None or g.numel() == 0:
             continue
         shards.append(g)
-        part = g.detach().float().abs().max() if inf else g.detach().float().norm(norm_type).pow(norm_type)
+        part = power_sum(g)
         group = u.groups.shard_group if u.world_size > 1 else None
         key = id(group)
         if key in per_group:
@@ -93,8 +108,7 @@ def clip_grad_norm_(module_or_units, max_norm: float, norm_type: float = 2.0,
     extra_grads = list(extra_grads)
     extra = [g for g in extra_grads if g is not None and g.numel()]
     if extra_grads:                  # also a rank whose experts saw no token joins the group's sum
-        parts = [g.detach().float().abs().max() if inf else g.detach().float().norm(norm_type).pow(norm_type)
-                 for g in extra]
+        parts = [power_sum(g) for g in extra]
         ref = shards[0] if shards else (extra[0] if extra else None)
         part = (torch.stack(parts).max() if inf else torch.stack(parts).sum()) if parts else \
             torch.zeros((), device=ref.device if ref is not None else None)
@@ -112,7 +126,11 @@ def clip_grad_norm_(module_or_units, max_norm: float, norm_type: float = 2.0,
         raise RuntimeError(f"The total norm of order {norm_type} for the gradients is non-finite.")
     coef = (max_norm / (norm + 1e-6)).clamp(max=1.0)
     for g in (*shards, *extra):
-        g.mul_(coef.to(device=g.device, dtype=g.dtype))
+        K = kernels_for(g) if coef.device == g.device and coef.dtype == torch.float32 else None
+        if K is not None:
+            K.scale_(g, coef)
+        else:
+            g.mul_(coef.to(device=g.device, dtype=g.dtype))
     return norm
 
 

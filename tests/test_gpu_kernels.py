@@ -455,13 +455,16 @@ def test_embedding_backward_orders_positions(K, T, V, H, ids):
     assert ((outs[0].double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -23 * T * size).all()
 
 
-@pytest.mark.parametrize("n,shift,f", [(1, 0, 0.5), (7, 0, -3.0), (4103, 0, 0.3), (4096, 1, 0.3), (4096, 0, 1.0)])
-def test_scale_bf16(K, n, shift, f):
-    """One fp32 product and one rounding per element: exact against the same in torch."""
-    x = torch.randn(n + shift, device="cuda").bfloat16()[shift:]
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,shift,f", [(1, 0, 0.5), (7, 0, -3.0), (4103, 0, 0.3), (4096, 1, 0.3), (4096, 0, 1.0), (3 << 20, 0, 0.7)])
+def test_scale_and_sum_of_squares(K, n, shift, f, dtype):
+    """One fp32 product and one rounding per element: exact against the same in torch.  The sum of n squares in fp32,
+    a few hundred terms per thread: 1e-5."""
+    x = torch.randn(n + shift, device="cuda").to(dtype)[shift:]
     s = torch.tensor(f, device="cuda")
-    want = (x.float() * s).bfloat16()
-    assert torch.equal(K.scale_bf16_(x, s), want)
+    total, want = x.double().pow(2).sum(), (x.float() * s).to(dtype)
+    assert (K.sumsq(x).double() - total).abs() <= 1e-5 * total
+    assert torch.equal(K.scale_(x, s), want)
 
 
 @pytest.mark.parametrize("rows,V,pad", [(1, 8, 0), (5, 1016, 8), (700, 1032, 0), (149, 4104, 0), (450, 16392, 0), (300, 32760, 8), (297, 49152, 0)])
