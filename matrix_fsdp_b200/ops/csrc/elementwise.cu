@@ -354,13 +354,17 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dh,
 }
 
 // ============================================================== cross-entropy
-// One CTA (128 to 1024 threads) per row keeps the whole row in registers (V <= threads*8*VPT):
+// One CTA (128 to 512 threads) per row keeps the whole row in registers, as the bf16 pairs it came in (V <= threads*8*VPT):
 // loss[row] = logsumexp - logit[target]; logits are overwritten with
 // (softmax - onehot) * grad_scale, i.e. the gradient of the mean loss.  When `grad_scale_dev` is
 // given the scale is read from device memory (1 / number of counted targets, computed on the device),
 // so a caller that masks targets needs no device-to-host read to launch this.
-template <int VPT>
-__global__ void __launch_bounds__(1024)
+// A row passes through phases (load, maximum, sum, store) that each leave most of the SM idle, so several rows have to
+// share it: packed values and taking the exponentials twice leave room for two blocks of 512 threads, where 1024 threads
+// with fp32 values ran alone: 16384 rows of 32000 logits 582 -> 416 us (5.0 TB/s), 3000 117 -> 86 us, 2048 rows of 8192
+// 30.7 -> 20.5 us, 16384 rows of 1024 131 -> 20.5 us.
+template <int VPT, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 cross_entropy_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ target,
                              float* __restrict__ loss, int V, long long ld, float grad_scale,
                              const float* __restrict__ grad_scale_dev, long long ignore_index) {
@@ -369,53 +373,63 @@ cross_entropy_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const long long
   const long long row = blockIdx.x;
   __nv_bfloat16* lr = logits + row * ld;
   const int nvec = V >> 3;
-  float f[VPT][8];
+  const long long tgt = target[row];
+  const bool valid = (tgt != ignore_index) && tgt >= 0 && tgt < V;
+  uint4 x[VPT];
   float mx = -INFINITY;
+  // one vector at a time, and nothing unpacked kept for the next phase: the registers have to do for two blocks
+  auto in_turn = [&](int i, float& acc) {
+    asm volatile("" : "+f"(acc), "+r"(x[i].x), "+r"(x[i].y), "+r"(x[i].z), "+r"(x[i].w));
+  };
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
-    const int v = threadIdx.x + i * blockDim.x;
+    const int v = threadIdx.x + i * THREADS;
+    x[i] = v < nvec ? reinterpret_cast<const uint4*>(lr)[v] : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);   // -inf
+  }
+  const float tgt_logit = threadIdx.x == 0 && valid ? __bfloat162float(lr[tgt]) : 0.f;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    in_turn(i, mx);
+    const uint32_t w[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 a = unpack_bf16x2(w[e]);
+      mx = fmaxf(mx, fmaxf(a.x, a.y));
+    }
+  }
+  mx = block_max(mx, red);      // its barriers also stand between the reading of the target's logit and the first store
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    in_turn(i, sum);
+    const uint32_t w[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 a = unpack_bf16x2(w[e]);
+      sum += __expf(a.x - mx) + __expf(a.y - mx);
+    }
+  }
+  sum = block_sum(sum, red);
+  if (threadIdx.x == 0) loss[row] = valid ? logf(sum) + mx - tgt_logit : 0.f;
+  float inv = valid ? grad_scale / sum : 0.f;
+  const int tgt_vec = valid ? (int)(tgt >> 3) : -1, tgt_elem = (int)(tgt & 7);
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int v = threadIdx.x + i * THREADS;
+    in_turn(i, inv);
     if (v < nvec) {
-      const uint4 u = reinterpret_cast<const uint4*>(lr)[v];
-      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+      const uint32_t w[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+      float o[8];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float2 a = unpack_bf16x2(w[e]);
-        f[i][2 * e] = a.x; f[i][2 * e + 1] = a.y;
-        mx = fmaxf(mx, fmaxf(a.x, a.y));
+        o[2 * e] = __expf(a.x - mx) * inv;
+        o[2 * e + 1] = __expf(a.y - mx) * inv;
       }
-    } else {
+      if (v == tgt_vec) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) f[i][e] = -INFINITY;
-    }
-  }
-  mx = block_max(mx, red);
-  float sum = 0.f;
-#pragma unroll
-  for (int i = 0; i < VPT; ++i)
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      f[i][e] = __expf(f[i][e] - mx);
-      sum += f[i][e];
-    }
-  sum = block_sum(sum, red);
-  const long long tgt = target[row];
-  const bool valid = (tgt != ignore_index) && tgt >= 0 && tgt < V;
-  if (threadIdx.x == 0) {
-    float l = 0.f;
-    if (valid) l = logf(sum) + mx - __bfloat162float(lr[tgt]);
-    loss[row] = l;
-  }
-  __syncthreads();  // the target logit is read above before any thread overwrites the row
-  const float inv = valid ? grad_scale / sum : 0.f;
-#pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int v = threadIdx.x + i * blockDim.x;
-    if (v < nvec) {
-      float o[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        o[e] = f[i][e] * inv;
-        if (valid && (long long)(v * 8 + e) == tgt) o[e] -= grad_scale;
+        for (int e = 0; e < 8; ++e)
+          if (e == tgt_elem) o[e] -= grad_scale;
       }
       reinterpret_cast<uint4*>(lr)[v] = make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]),
                                                    pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
@@ -1032,20 +1046,23 @@ static int launch_cross_entropy(void* logits, const long long* target, float* lo
                                 long long ld, float grad_scale, const float* grad_scale_dev,
                                 long long ignore_index, cudaStream_t st) {
   if (V % 8 || ld % 8) return -2;
-  // as few threads as hold the row in four vectors each: short rows then share an SM instead of idling most of a block
-  // (16384 rows of 1024 logits: 131 us with 1024 threads, 35 with 128); rows through a ring of shared-memory buffers
-  // with bulk copies were no faster at 32000 logits (596 against 582 us for 16384 rows: the arithmetic bounds it)
+  // as few threads as hold the row in eight vectors each (twelve above 32768 logits): short rows then share an SM instead
+  // of idling most of a block.  Rows through a ring of shared-memory buffers with bulk copies were no faster (16384 rows of
+  // 32000: 596 us, against 582 of 1024 threads with their row in fp32 registers).
   const int nvec = V / 8;
-  int threads = 128;
-  while (threads < 1024 && nvec > 4 * threads) threads *= 2;
-  const int vpt = (nvec + threads - 1) / threads;
   auto L = (__nv_bfloat16*)logits;
   const unsigned g = (unsigned)rows;
-  if (vpt <= 1) cross_entropy_fwd_bwd_kernel<1><<<g, threads, 0, st>>>(L, target, loss, V, ld, grad_scale, grad_scale_dev, ignore_index);
-  else if (vpt <= 2) cross_entropy_fwd_bwd_kernel<2><<<g, threads, 0, st>>>(L, target, loss, V, ld, grad_scale, grad_scale_dev, ignore_index);
-  else if (vpt <= 4) cross_entropy_fwd_bwd_kernel<4><<<g, threads, 0, st>>>(L, target, loss, V, ld, grad_scale, grad_scale_dev, ignore_index);
-  else if (vpt <= 6) cross_entropy_fwd_bwd_kernel<6><<<g, threads, 0, st>>>(L, target, loss, V, ld, grad_scale, grad_scale_dev, ignore_index);
+#define MFSDP_CE(VPT, THREADS) \
+  cross_entropy_fwd_bwd_kernel<VPT, THREADS><<<g, THREADS, 0, st>>>(L, target, loss, V, ld, grad_scale, grad_scale_dev, ignore_index)
+  if (nvec <= 128) MFSDP_CE(1, 128);
+  else if (nvec <= 256) MFSDP_CE(2, 128);
+  else if (nvec <= 512) MFSDP_CE(4, 128);
+  else if (nvec <= 1024) MFSDP_CE(4, 256);
+  else if (nvec <= 2048) MFSDP_CE(8, 256);
+  else if (nvec <= 4096) MFSDP_CE(8, 512);
+  else if (nvec <= 6144) MFSDP_CE(12, 512);
   else return -2;
+#undef MFSDP_CE
   return (int)cudaGetLastError();
 }
 
