@@ -126,6 +126,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs p
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_begin();
   const uint32_t tmem_o = tmem_base + 256;
   const uint32_t sQ = smem_u32(smem + AttnFwdSmem::kQ), sK = smem_u32(smem + AttnFwdSmem::kK),
                  sV = smem_u32(smem + AttnFwdSmem::kV), sP = smem_u32(smem + AttnFwdSmem::kP);
@@ -370,6 +371,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_begin();
   const uint32_t sQ = smem_u32(smem + AttnFwd2Smem::kQ), sK = smem_u32(smem + AttnFwd2Smem::kK),
                  sV = smem_u32(smem + AttnFwd2Smem::kV);
 
@@ -649,6 +651,7 @@ __device__ __forceinline__ void attn_bwd_block(const CUtensorMap& tma_qkv, const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_begin();
   const uint32_t tmem_dp = tmem_base + 128, tmem_acc0 = tmem_base + 256, tmem_acc1 = tmem_base + 384;
   const uint32_t sA0 = smem_u32(smem + AttnBwdSmem::kA0), sA1 = smem_u32(smem + AttnBwdSmem::kA1),
                  sB = smem_u32(smem + AttnBwdSmem::kB);
@@ -860,6 +863,7 @@ attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ dout, long long ld_do, co
                      int B, int S, int nH, int Sp) {
   const long long w = (long long)blockIdx.x * 16 + (threadIdx.x >> 4);
   const int lane = threadIdx.x & 15;
+  pdl_begin();
   if (w >= (long long)B * Sp * nH) return;                 // whole half-warps leave
   const int hh = (int)(w % nH);
   const long long row = w / nH;
@@ -924,12 +928,11 @@ MFSDP_API int mfsdp_attention_fwd(const void* qkv, void* out, float* lse, int B,
   a.out = (__nv_bfloat16*)out; a.ld_out = ld_out; a.lse = lse; a.status = status;
   if (attn_fwd_two_tiles(B, S, nH)) {
     const int nq = (S + 2 * kBq - 1) / (2 * kBq);
-    attn_fwd2_kernel<<<(unsigned)(nq * B * nH), kFwd2Threads, AttnFwd2Smem::kBytes, st>>>(map, a, heads_in_l2(B, S, nH));
-    return (int)cudaGetLastError();
+    return launch_pdl(attn_fwd2_kernel, dim3((unsigned)(nq * B * nH)), dim3(kFwd2Threads), AttnFwd2Smem::kBytes, st, map, a,
+                      heads_in_l2(B, S, nH));
   }
   dim3 grid((S + kBq - 1) / kBq, nH, B);
-  attn_fwd_kernel<<<grid, kAttnThreads, AttnFwdSmem::kBytes, st>>>(map, a);
-  return (int)cudaGetLastError();
+  return launch_pdl(attn_fwd_kernel, grid, dim3(kAttnThreads), AttnFwdSmem::kBytes, st, map, a);
 }
 
 // dout, out: [B*S, nH*128] bf16; lse: [B, nH, S]; dqkv: [B*S, 3*nH*128] bf16 (written in full);
@@ -956,12 +959,13 @@ MFSDP_API int mfsdp_attention_bwd(const void* dout, const void* qkv, const void*
   a.Sp = (long long)nt * 128;
   float* nlse2 = scratch;
   float* ndelta = scratch + (long long)B * nH * a.Sp;
-  attn_bwd_prep_kernel<<<(unsigned)(((long long)B * nH * a.Sp + 15) / 16), 256, 0, st>>>(
-      (const __nv_bfloat16*)dout, ld_o, (const __nv_bfloat16*)out, ld_o, lse, nlse2, ndelta, B, S, nH, (int)a.Sp);
+  rc = launch_pdl(attn_bwd_prep_kernel, dim3((unsigned)(((long long)B * nH * a.Sp + 15) / 16)), dim3(256), 0, st,
+                  (const __nv_bfloat16*)dout, ld_o, (const __nv_bfloat16*)out, ld_o, lse, nlse2, ndelta, B, S, nH, (int)a.Sp);
+  if (rc) return rc;
   a.scale = softmax_scale; a.scale_log2 = softmax_scale * kLog2e;
   a.nlse2 = nlse2; a.ndelta = ndelta;
   a.dqkv = (__nv_bfloat16*)dqkv; a.ld_dqkv = ld_dqkv; a.status = status;
   a.heads_per_group = heads_in_l2(B, S, nH);
-  attn_bwd_kernel<<<2u * (unsigned)(nt * B * nH), kBwdThreads, AttnBwdSmem::kBytes, st>>>(map_qkv, map_do, a);
-  return (int)cudaGetLastError();
+  return launch_pdl(attn_bwd_kernel, dim3(2u * (unsigned)(nt * B * nH)), dim3(kBwdThreads), AttnBwdSmem::kBytes, st, map_qkv,
+                    map_do, a);
 }

@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(256)
 rmsnorm_fwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                         __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, long long rows, int H, float eps) {
   __shared__ float part[8];
+  pdl_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * (8 / WPR) + warp / WPR;
   const int first = (warp % WPR) * 32 + lane, nvec = H >> 3;
@@ -137,6 +138,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   constexpr int RPC = 8 / WPR;
   __shared__ float part[2][8];
   extern __shared__ float dw_smem[];          // [H]
+  pdl_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, slot = warp / WPR;
   const int first = (warp % WPR) * 32 + lane, nvec = H >> 3;
   float dwp[VPL][8];
@@ -238,6 +240,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 __global__ void colsum_f32_to_bf16_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out,
                                           int rows, int H, int accumulate) {
   __shared__ float tile[8][33];
+  pdl_begin();
   const int col = blockIdx.x * 32 + threadIdx.x;
   float acc = 0.f;
   if (col < H)
@@ -260,6 +263,7 @@ __global__ void colsum_f32_to_bf16_kernel(const float* __restrict__ partial, __n
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, long long T, int S, int ld, int col0,
                             int n_heads, int D, float sign) {
+  pdl_begin();
   const int half = D >> 1;
   const int vec_per_head = half >> 3;  // 8 bf16 per vector
   const long long total = T * (long long)n_heads * vec_per_head;
@@ -300,6 +304,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __rest
 // gu is [T, 2F]: gate in columns [0,F), up in [F,2F).  h = silu(gate) * up.
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h,
                                   long long T, int F) {
+  pdl_begin();
   const int vpr = F >> 3;
   const long long total = T * vpr;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -325,6 +330,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dh,
                                   const __nv_bfloat16* __restrict__ gu,
                                   __nv_bfloat16* __restrict__ dgu, long long T, int F) {
+  pdl_begin();
   const int vpr = F >> 3;
   const long long total = T * vpr;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -369,6 +375,7 @@ cross_entropy_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const long long
                              float* __restrict__ loss, int V, long long ld, float grad_scale,
                              const float* __restrict__ grad_scale_dev, long long ignore_index) {
   __shared__ float red[32];
+  pdl_begin();
   if (grad_scale_dev != nullptr) grad_scale = *grad_scale_dev;
   const long long row = blockIdx.x;
   __nv_bfloat16* lr = logits + row * ld;
@@ -959,8 +966,8 @@ MFSDP_API int mfsdp_rmsnorm_fwd(const void* x, const void* w, void* y, float* rs
                      nvec <= 256 ? rmsnorm_fwd_rows_kernel<8, 1> : nvec <= 512 ? rmsnorm_fwd_rows_kernel<8, 2> :
                      nvec <= 1024 ? rmsnorm_fwd_rows_kernel<8, 4> : rmsnorm_fwd_rows_kernel<8, 8>;
   const int rpc = nvec <= 256 ? 8 : nvec <= 512 ? 4 : nvec <= 1024 ? 2 : 1;
-  if (nvec <= 2048) rows_kernel<<<(unsigned)((rows + rpc - 1) / rpc), 256, 0, st>>>(X, W, Y, rstd, rows, H, eps);
-  else if (nvec <= 8 * 1024) rmsnorm_fwd_kernel<8><<<(unsigned)rows, 1024, 0, st>>>(X, W, Y, rstd, H, eps);
+  if (nvec <= 2048) return launch_pdl(rows_kernel, dim3((unsigned)((rows + rpc - 1) / rpc)), dim3(256), 0, st, X, W, Y, rstd, rows, H, eps);
+  if (nvec <= 8 * 1024) rmsnorm_fwd_kernel<8><<<(unsigned)rows, 1024, 0, st>>>(X, W, Y, rstd, H, eps);
   else return -2;
   return (int)cudaGetLastError();
 }
@@ -980,7 +987,7 @@ static int launch_rmsnorm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* x, c
   const int grid = (int)((groups + trips - 1) / trips);
   auto kern = nvec <= 64 ? rmsnorm_bwd_kernel<2, 1> : nvec <= 128 ? rmsnorm_bwd_kernel<4, 1> :
               nvec <= 256 ? rmsnorm_bwd_kernel<4, 2> : nvec <= 512 ? rmsnorm_bwd_kernel<4, 4> : rmsnorm_bwd_kernel<4, 8>;
-  kern<<<grid, 256, H * sizeof(float), st>>>(dy, x, w, rstd, dres, dx, dw_acc, rows, H);
+  launch_pdl(kern, dim3(grid), dim3(256), H * sizeof(float), st, dy, x, w, rstd, dres, dx, dw_acc, rows, H);
   return grid;
 }
 
@@ -993,7 +1000,7 @@ MFSDP_API int mfsdp_rmsnorm_bwd(const void* dy, const void* x, const void* w, co
   if (rows <= 0) return -2;
   const int grid = launch_rmsnorm_bwd((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
                                       (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw_acc, rows, H, kRmsBwdCtas, st);
-  if (dw) colsum_f32_to_bf16_kernel<<<(H + 31) / 32, dim3(32, 8), 0, st>>>(dw_acc, (__nv_bfloat16*)dw, grid, H, accumulate_dw);
+  if (dw) launch_pdl(colsum_f32_to_bf16_kernel, dim3((H + 31) / 32), dim3(32, 8), 0, st, dw_acc, (__nv_bfloat16*)dw, grid, H, accumulate_dw);
   return (int)cudaGetLastError();
 }
 
@@ -1001,16 +1008,13 @@ MFSDP_API int mfsdp_rope(void* qkv, const float* cos_t, const float* sin_t, long
                          int col0, int n_heads, int D, float sign, cudaStream_t st) {
   if (D % 16 || ld % 8 || col0 % 8) return -2;
   const long long work = T * (long long)n_heads * (D / 16);
-  rope_kernel<<<grid_for(work, 256, 148 * 16), 256, 0, st>>>((__nv_bfloat16*)qkv, cos_t, sin_t, T, S, ld, col0,
-                                                   n_heads, D, sign);
-  return (int)cudaGetLastError();
+  return launch_pdl(rope_kernel, dim3(grid_for(work, 256, 148 * 16)), dim3(256), 0, st, (__nv_bfloat16*)qkv, cos_t, sin_t, T, S, ld,
+                    col0, n_heads, D, sign);
 }
 
 MFSDP_API int mfsdp_swiglu_fwd(const void* gu, void* h, long long T, int F, cudaStream_t st) {
   if (F % 8) return -2;
-  swiglu_fwd_kernel<<<grid_for(T * (F / 8), 256, 148 * 16), 256, 0, st>>>((const __nv_bfloat16*)gu,
-                                                                 (__nv_bfloat16*)h, T, F);
-  return (int)cudaGetLastError();
+  return launch_pdl(swiglu_fwd_kernel, dim3(grid_for(T * (F / 8), 256, 148 * 16)), dim3(256), 0, st, (const __nv_bfloat16*)gu, (__nv_bfloat16*)h, T, F);
 }
 
 // dW[V, H] (row pitch lddw) from dy[T, H] (row pitch lddy) and ids[T]; `work` holds 2 * V + 2 * T + 1 ints.  Ids outside
@@ -1037,9 +1041,7 @@ MFSDP_API int mfsdp_embedding_bwd(const void* dy, long long lddy, const long lon
 MFSDP_API int mfsdp_swiglu_bwd(const void* dh, const void* gu, void* dgu, long long T, int F,
                                cudaStream_t st) {
   if (F % 8) return -2;
-  swiglu_bwd_kernel<<<grid_for(T * (F / 8), 256, 148 * 16), 256, 0, st>>>(
-      (const __nv_bfloat16*)dh, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, T, F);
-  return (int)cudaGetLastError();
+  return launch_pdl(swiglu_bwd_kernel, dim3(grid_for(T * (F / 8), 256, 148 * 16)), dim3(256), 0, st, (const __nv_bfloat16*)dh, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, T, F);
 }
 
 static int launch_cross_entropy(void* logits, const long long* target, float* loss, long long rows, int V,
@@ -1053,17 +1055,17 @@ static int launch_cross_entropy(void* logits, const long long* target, float* lo
   auto L = (__nv_bfloat16*)logits;
   const unsigned g = (unsigned)rows;
 #define MFSDP_CE(VPT, THREADS) \
-  cross_entropy_fwd_bwd_kernel<VPT, THREADS><<<g, THREADS, 0, st>>>(L, target, loss, V, ld, grad_scale, grad_scale_dev, ignore_index)
+  return launch_pdl(cross_entropy_fwd_bwd_kernel<VPT, THREADS>, dim3(g), dim3(THREADS), 0, st, L, target, loss, V, ld, grad_scale, \
+                    grad_scale_dev, ignore_index)
   if (nvec <= 128) MFSDP_CE(1, 128);
-  else if (nvec <= 256) MFSDP_CE(2, 128);
-  else if (nvec <= 512) MFSDP_CE(4, 128);
-  else if (nvec <= 1024) MFSDP_CE(4, 256);
-  else if (nvec <= 2048) MFSDP_CE(8, 256);
-  else if (nvec <= 4096) MFSDP_CE(8, 512);
-  else if (nvec <= 6144) MFSDP_CE(12, 512);
-  else return -2;
+  if (nvec <= 256) MFSDP_CE(2, 128);
+  if (nvec <= 512) MFSDP_CE(4, 128);
+  if (nvec <= 1024) MFSDP_CE(4, 256);
+  if (nvec <= 2048) MFSDP_CE(8, 256);
+  if (nvec <= 4096) MFSDP_CE(8, 512);
+  if (nvec <= 6144) MFSDP_CE(12, 512);
 #undef MFSDP_CE
-  return (int)cudaGetLastError();
+  return -2;
 }
 
 MFSDP_API int mfsdp_cross_entropy(void* logits, const long long* target, float* loss, long long rows,
@@ -1271,6 +1273,6 @@ MFSDP_API int mfsdp_rmsnorm_bwd_noalloc(const void* dy, const void* x, const voi
   }
   const int grid = launch_rmsnorm_bwd((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
                                       (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, H, MFSDP_NOALLOC_SCRATCH_ROWS, st);
-  if (dw) colsum_f32_to_bf16_kernel<<<(H + 31) / 32, dim3(32, 8), 0, st>>>(scratch, (__nv_bfloat16*)dw, grid, H, accumulate_dw);
+  if (dw) launch_pdl(colsum_f32_to_bf16_kernel, dim3((H + 31) / 32), dim3(32, 8), 0, st, scratch, (__nv_bfloat16*)dw, grid, H, accumulate_dw);
   return (int)cudaGetLastError();
 }

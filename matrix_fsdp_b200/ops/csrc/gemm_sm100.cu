@@ -232,6 +232,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_begin();
 
   const int total_tiles = p.total_tiles;
 
@@ -596,8 +597,11 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
-  kern<<<grid, GATHER ? kGemmThreads + kGatherThreads : kGemmThreads, Cfg::kSmemBytes, stream>>>(ta, tb, td, tt, args);
-  return (int)cudaGetLastError();
+  if (GATHER) {                            // reads flags that peers and other streams set: launched in plain stream order
+    kern<<<grid, kGemmThreads + kGatherThreads, Cfg::kSmemBytes, stream>>>(ta, tb, td, tt, args);
+    return (int)cudaGetLastError();
+  }
+  return launch_pdl(kern, dim3(grid), dim3(kGemmThreads), Cfg::kSmemBytes, stream, ta, tb, td, tt, args);
 }
 
 // CTA-pair kernels are launched as clusters of two; the persistent grid is as many pairs as can be
@@ -609,7 +613,9 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const 
   auto kern = gemm_bf16_tcgen05_kernel<256, A_MN, B_MN, false, true>;
   static int max_pairs = -1;
   cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -632,6 +638,7 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const 
   int pairs = args.total_tiles < max_pairs ? args.total_tiles : max_pairs;
   if (pairs > num_sms / 2) pairs = num_sms / 2;
   cfg.gridDim = dim3((unsigned)(2 * pairs));
+  cfg.numAttrs = 2;
   return (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, td, tt, args);
 }
 
