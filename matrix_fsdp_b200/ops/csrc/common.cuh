@@ -369,6 +369,12 @@ __device__ __forceinline__ float2 unpack_bf16x2(uint32_t u) {
   __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&u);
   return __bfloat1622float2(v);
 }
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
+  const uint4 u = *reinterpret_cast<const uint4*>(p);
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) { const float2 v = unpack_bf16x2(w[e]); f[2 * e] = v.x; f[2 * e + 1] = v.y; }
+}
 // Two fp32 values in one register pair: one instruction for both (sm_100), each rounded as usual.
 __device__ __forceinline__ uint64_t pack_u32x2(uint32_t lo, uint32_t hi) {
   uint64_t d;

@@ -511,3 +511,20 @@ def test_rmsnorm_rows_and_widths(K, rows, H):
         assert _rel_err(dx, xd.grad + (res.double() if res is not None else 0)) < 2 ** -7
         assert _rel_err(acc, wd.grad + (old.double() if res is None else 0)) < 2 ** -7
         assert dw is acc
+
+
+@pytest.mark.parametrize("M,N,Kd,shift,pitch", [(200, 72, 64, 0, 72), (256, 264, 128, 0, 272), (300, 320, 64, 3, 331), (513, 1000, 192, 8, 1016)])
+def test_gemm_adds_cin_of_any_pitch(K, M, N, Kd, shift, pitch):
+    """Whole 64-column chunks by vectors read ahead, the right edge and rows off the 16-byte grid element by element, and
+    Cin that is the output itself.  Bound: one bf16 rounding of an fp32 sum."""
+    torch.manual_seed(M)
+    a, b = _rand(M, Kd, scale=Kd ** -0.5), _rand(N, Kd)
+    c = torch.randn(M * pitch + shift, device="cuda").bfloat16()[shift:].as_strided((M, N), (pitch, 1))
+    want = 0.5 * (a.double() @ b.double().t()) - 2.0 * c.double()
+    for force in (0, 2, 128, 256):
+        out = K.gemm(a, b, cin=c, alpha=0.5, beta=-2.0, force_bn=force)
+        assert _rel_err(out, want) < 2 ** -8, force
+    inplace = c.contiguous()
+    K.gemm(a, b, cin=inplace, out=inplace, alpha=0.5, beta=-2.0)
+    assert _rel_err(inplace, want) < 2 ** -8
+    K.check_status()
