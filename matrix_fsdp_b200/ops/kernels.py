@@ -429,10 +429,14 @@ def cast_bf16_f32(src: torch.Tensor, dst: torch.Tensor) -> None:
 
 
 def scale_(x: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:
-    """``x *= scale`` for a contiguous bf16 or fp32 tensor and a one-element fp32 device tensor (no host read)."""
+    """``x *= scale`` for a contiguous bf16 or fp32 tensor and a one-element fp32 device tensor (no host read).
+
+    Counts as an in-place operation for autograd, like ``x.mul_(scale)``: a graph that saved ``x`` refuses to be walked
+    again instead of reading the scaled values."""
     assert x.dtype in (torch.bfloat16, torch.float32) and x.is_contiguous()
     assert scale.dtype == torch.float32 and scale.numel() == 1 and scale.device == x.device
     _lib.check(_L().mfsdp_scale(x.data_ptr(), int(x.dtype == torch.bfloat16), x.numel(), scale.data_ptr(), _stream()), "scale")
+    torch.autograd.graph.increment_version(x)
     return x
 
 

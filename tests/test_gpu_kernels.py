@@ -528,3 +528,21 @@ def test_gemm_adds_cin_of_any_pitch(K, M, N, Kd, shift, pitch):
     K.gemm(a, b, cin=inplace, out=inplace, alpha=0.5, beta=-2.0)
     assert _rel_err(inplace, want) < 2 ** -8
     K.check_status()
+
+
+@pytest.mark.parametrize("factor", [0.5, 1.0])
+def test_scaled_cross_entropy_is_walked_once(factor):
+    """The gradient lies in the logits buffer and takes the upstream factor there: the first walk is right (two bf16
+    roundings), a second over a kept graph is refused."""
+    from matrix_fsdp_b200.ops import functional as OF
+
+    torch.manual_seed(0)
+    logits = _rand(65, 1000).requires_grad_(True)
+    target = torch.randint(0, 1000, (65,), device="cuda")
+    loss = OF.fused_cross_entropy(logits * 1, target) * factor
+    (grad,) = torch.autograd.grad(loss, logits, retain_graph=True)
+    x = logits.detach().double().requires_grad_(True)
+    (want,) = torch.autograd.grad(torch.nn.functional.cross_entropy(x, target) * factor, x)
+    assert ((grad.double() - want).abs() <= 2 ** -7 * want.abs() + 1e-9).all()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(loss, logits)
