@@ -423,9 +423,11 @@ def cast_f32_bf16(src: torch.Tensor, dst: torch.Tensor) -> None:
 
 
 def cast_bf16_f32(src: torch.Tensor, dst: torch.Tensor) -> None:
+    """``dst = src``, recorded for autograd like the ``copy_`` it stands for."""
     assert src.dtype == torch.bfloat16 and dst.dtype == torch.float32 and src.numel() == dst.numel()
     assert src.is_contiguous() and dst.is_contiguous()
     _lib.check(_L().mfsdp_cast_bf16_f32(src.data_ptr(), dst.data_ptr(), src.numel(), _stream()), "cast_bf16_f32")
+    torch.autograd.graph.increment_version(dst)
 
 
 def scale_(x: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:

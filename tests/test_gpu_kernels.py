@@ -546,3 +546,16 @@ def test_scaled_cross_entropy_is_walked_once(factor):
     assert ((grad.double() - want).abs() <= 2 ** -7 * want.abs() + 1e-9).all()
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         torch.autograd.grad(loss, logits)
+
+
+def test_adamw_records_the_low_precision_copy_for_autograd():
+    from matrix_fsdp_b200.optim.flat import FlatShardedAdamW
+
+    p = torch.nn.Parameter(torch.randn(64, device="cuda"))
+    p.grad = torch.randn(64, device="cuda")
+    shard = torch.zeros(128, device="cuda", dtype=torch.bfloat16)
+    opt = FlatShardedAdamW([p], lr=1e-2)
+    opt._low_precision_of = lambda _: shard[64:]
+    version = shard._version
+    opt.step()
+    assert torch.equal(shard[64:], p.detach().bfloat16()) and shard._version > version

@@ -26,6 +26,11 @@ class _Library:
         return 0
 
     @staticmethod
+    def mfsdp_cast_bf16_f32(src, dst, n, stream):
+        _memory(dst, (n,), torch.float32).copy_(_memory(src, (n,), torch.bfloat16))
+        return 0
+
+    @staticmethod
     def mfsdp_cross_entropy_dev_scale(logits, target, loss, rows, V, ld, scale, ignore_index, stream):
         assert ld == V
         x = _memory(logits, (rows, V), torch.bfloat16)
@@ -52,6 +57,17 @@ def test_scaling_in_place_is_seen_by_autograd(library, dtype):
     version = base._version
     assert torch.equal(K.scale_(base[8:], torch.tensor(0.5)), want)
     assert base._version > version
+
+
+def test_widening_copy_is_seen_by_autograd(library):
+    """A graph that saved the destination (a slice of a gradient shard) must not be walked over the new values."""
+    src, shard = torch.randn(16).bfloat16(), torch.randn(24)
+    w = torch.randn(16, requires_grad=True)
+    y = (w * shard[8:]).sum()
+    K.cast_bf16_f32(src, shard[8:])
+    assert torch.equal(shard[8:], src.float())
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.backward()
 
 
 def test_a_scaled_loss_is_not_walked_twice_over_one_graph(library):
