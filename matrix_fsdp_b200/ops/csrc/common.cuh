@@ -440,4 +440,46 @@ __device__ __forceinline__ float block_max(float v, float* red) {
   return red[0];
 }
 
+// ---------------------------------------------------------------- AdamW
+// Constants of one AdamW step, each computed in 64 bits on the host and rounded once: 1 - beta2 = 1e-3 as the difference
+// of two fp32 numbers would be 1.3e-5 off, and so would the bias correction from an fp32 power.
+struct AdamWStep {
+  float keep;                    // 1 - lr * weight_decay
+  float beta1, one_minus_beta1, beta2, one_minus_beta2;
+  float eps, bias2_sqrt;         // sqrt(1 - beta2^step)
+  float step_size;               // lr / (1 - beta1^step)
+  float grad_scale;
+};
+
+inline AdamWStep adamw_step(double lr, double beta1, double beta2, double eps, double weight_decay, long long step,
+                            double grad_scale) {
+  AdamWStep a;
+  a.keep = (float)(1.0 - lr * weight_decay);
+  a.beta1 = (float)beta1;
+  a.one_minus_beta1 = (float)(1.0 - beta1);
+  a.beta2 = (float)beta2;
+  a.one_minus_beta2 = (float)(1.0 - beta2);
+  a.eps = (float)eps;
+  a.bias2_sqrt = (float)sqrt(1.0 - pow(beta2, (double)step));
+  a.step_size = (float)(lr / (1.0 - pow(beta1, (double)step)));
+  a.grad_scale = (float)grad_scale;
+  return a;
+}
+
+// The rounding of torch's fp32 operations whatever --use_fast_math makes of the operators: correctly rounded square root
+// and quotients, and small moments kept below the normal range (fast math flushes them).
+__device__ __forceinline__ float ieee_mul(float a, float b) { float d; asm("mul.rn.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b)); return d; }
+__device__ __forceinline__ float ieee_add(float a, float b) { float d; asm("add.rn.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b)); return d; }
+__device__ __forceinline__ float ieee_fma(float a, float b, float c) { float d; asm("fma.rn.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
+__device__ __forceinline__ float ieee_div(float a, float b) { float d; asm("div.rn.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b)); return d; }
+__device__ __forceinline__ float ieee_sqrt(float a) { float d; asm("sqrt.rn.f32 %0, %1;" : "=f"(d) : "f"(a)); return d; }
+
+__device__ __forceinline__ void adamw_update(float& p, float& m, float& v, float g, const AdamWStep& a) {
+  g = ieee_mul(g, a.grad_scale);
+  m = ieee_fma(a.beta1, m, ieee_mul(a.one_minus_beta1, g));
+  v = ieee_fma(a.beta2, v, ieee_mul(ieee_mul(a.one_minus_beta2, g), g));
+  const float denom = ieee_add(ieee_div(ieee_sqrt(v), a.bias2_sqrt), a.eps);
+  p = ieee_fma(-a.step_size, ieee_div(m, denom), ieee_mul(p, a.keep));
+}
+
 }  // namespace mfsdp

@@ -453,8 +453,7 @@ cross_entropy_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const long long
 template <typename GradT>
 __global__ void adamw_flat_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
                                   const GradT* __restrict__ g, __nv_bfloat16* __restrict__ p_lp,
-                                  long long n, float lr, float beta1, float beta2, float eps,
-                                  float weight_decay, float bias1, float bias2_sqrt, float grad_scale) {
+                                  long long n, const AdamWStep a) {
   const long long nv = n >> 2;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += stride) {
@@ -464,24 +463,17 @@ __global__ void adamw_flat_kernel(float* __restrict__ p, float* __restrict__ m, 
     float gg[4];
     if constexpr (sizeof(GradT) == 2) {
       const uint2 u = reinterpret_cast<const uint2*>(g)[i];
-      const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y);
-      gg[0] = a.x; gg[1] = a.y; gg[2] = b.x; gg[3] = b.y;
+      const float2 a2 = unpack_bf16x2(u.x), b2 = unpack_bf16x2(u.y);
+      gg[0] = a2.x; gg[1] = a2.y; gg[2] = b2.x; gg[3] = b2.y;
     } else {
-      const float4 a = reinterpret_cast<const float4*>(g)[i];
-      gg[0] = a.x; gg[1] = a.y; gg[2] = a.z; gg[3] = a.w;
+      const float4 g4 = reinterpret_cast<const float4*>(g)[i];
+      gg[0] = g4.x; gg[1] = g4.y; gg[2] = g4.z; gg[3] = g4.w;
     }
     float* pa = reinterpret_cast<float*>(&pp);
     float* ma = reinterpret_cast<float*>(&mm);
     float* va = reinterpret_cast<float*>(&vv);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float gr = gg[e] * grad_scale;
-      pa[e] *= (1.f - lr * weight_decay);
-      ma[e] = beta1 * ma[e] + (1.f - beta1) * gr;
-      va[e] = beta2 * va[e] + (1.f - beta2) * gr * gr;
-      const float denom = sqrtf(va[e]) / bias2_sqrt + eps;
-      pa[e] -= (lr / bias1) * (ma[e] / denom);
-    }
+    for (int e = 0; e < 4; ++e) adamw_update(pa[e], ma[e], va[e], gg[e], a);
     reinterpret_cast<float4*>(p)[i] = pp;
     reinterpret_cast<float4*>(m)[i] = mm;
     reinterpret_cast<float4*>(v)[i] = vv;
@@ -491,13 +483,11 @@ __global__ void adamw_flat_kernel(float* __restrict__ p, float* __restrict__ m, 
   // scalar tail
   for (long long i = (nv << 2) + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
     float gr;
-    if constexpr (sizeof(GradT) == 2) gr = __bfloat162float(g[i]) * grad_scale;
-    else gr = (float)g[i] * grad_scale;
-    float pv = p[i] * (1.f - lr * weight_decay);
-    const float mv = beta1 * m[i] + (1.f - beta1) * gr;
-    const float vv2 = beta2 * v[i] + (1.f - beta2) * gr * gr;
-    pv -= (lr / bias1) * (mv / (sqrtf(vv2) / bias2_sqrt + eps));
-    p[i] = pv; m[i] = mv; v[i] = vv2;
+    if constexpr (sizeof(GradT) == 2) gr = __bfloat162float(g[i]);
+    else gr = (float)g[i];
+    float pv = p[i], mv = m[i], vv = v[i];
+    adamw_update(pv, mv, vv, gr, a);
+    p[i] = pv; m[i] = mv; v[i] = vv;
     if (p_lp) p_lp[i] = __float2bfloat16_rn(pv);
   }
 }
@@ -1077,21 +1067,18 @@ MFSDP_API int mfsdp_cross_entropy_dev_scale(void* logits, const long long* targe
 }
 
 MFSDP_API int mfsdp_adamw_flat(float* p, float* m, float* v, const void* g, int grad_is_bf16, void* p_lp,
-                               long long n, float lr, float beta1, float beta2, float eps,
-                               float weight_decay, long long step, float grad_scale, cudaStream_t st) {
+                               long long n, double lr, double beta1, double beta2, double eps,
+                               double weight_decay, long long step, double grad_scale, cudaStream_t st) {
   if (n <= 0) return 0;
   if (((uintptr_t)p & 15) || ((uintptr_t)m & 15) || ((uintptr_t)v & 15) ||
       ((uintptr_t)g & (grad_is_bf16 ? 7 : 15)) || ((uintptr_t)p_lp & 7))
     return -2;
-  const float bias1 = 1.f - powf(beta1, (float)step);
-  const float bias2_sqrt = sqrtf(1.f - powf(beta2, (float)step));
+  const AdamWStep a = adamw_step(lr, beta1, beta2, eps, weight_decay, step, grad_scale);
   const int grid = grid_for(n / 4 + 1, 256, 148 * 8);
   if (grad_is_bf16)
-    adamw_flat_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p, m, v, (const __nv_bfloat16*)g, (__nv_bfloat16*)p_lp, n, lr,
-                                                           beta1, beta2, eps, weight_decay, bias1, bias2_sqrt, grad_scale);
+    adamw_flat_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p, m, v, (const __nv_bfloat16*)g, (__nv_bfloat16*)p_lp, n, a);
   else
-    adamw_flat_kernel<float><<<grid, 256, 0, st>>>(p, m, v, (const float*)g, (__nv_bfloat16*)p_lp, n, lr, beta1, beta2,
-                                                   eps, weight_decay, bias1, bias2_sqrt, grad_scale);
+    adamw_flat_kernel<float><<<grid, 256, 0, st>>>(p, m, v, (const float*)g, (__nv_bfloat16*)p_lp, n, a);
   return (int)cudaGetLastError();
 }
 

@@ -278,15 +278,8 @@ struct AdamWArgs {
   float* m;
   float* v;
   __nv_bfloat16* p_lp;
-  float lr, beta1, beta2, eps, weight_decay, bias1, bias2_sqrt;
+  AdamWStep step;
 };
-
-__device__ __forceinline__ void adamw_one(float& p, float& m, float& v, float g, const AdamWArgs& a) {
-  p *= (1.f - a.lr * a.weight_decay);
-  m = a.beta1 * m + (1.f - a.beta1) * g;
-  v = a.beta2 * v + (1.f - a.beta2) * g * g;
-  p -= (a.lr / a.bias1) * (m / (sqrtf(v) / a.bias2_sqrt + a.eps));
-}
 
 template <typename TIn, int WORLD>
 __global__ void rs_pull_adamw_kernel(PeerPtrs grads, int world_rt, int rank, ReduceTable tab, int nseg, float scale,
@@ -309,7 +302,7 @@ __global__ void rs_pull_adamw_kernel(PeerPtrs grads, int world_rt, int rank, Red
       load8(a.m + j, mm);
       load8(a.v + j, vv);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) adamw_one(pp[e], mm[e], vv[e], acc[e] * scale, a);
+      for (int e = 0; e < 8; ++e) adamw_update(pp[e], mm[e], vv[e], acc[e] * scale, a.step);
       store8(a.p + j, pp);
       store8(a.m + j, mm);
       store8(a.v + j, vv);
@@ -323,7 +316,7 @@ __global__ void rs_pull_adamw_kernel(PeerPtrs grads, int world_rt, int rank, Red
       }
       const long long j = l0 + i;
       float pp = a.p[j], mm = a.m[j], vv = a.v[j];
-      adamw_one(pp, mm, vv, acc * scale, a);
+      adamw_update(pp, mm, vv, acc * scale, a.step);
       a.p[j] = pp; a.m[j] = mm; a.v[j] = vv;
       if (a.p_lp) a.p_lp[j] = __float2bfloat16_rn(pp);
     }
@@ -484,7 +477,7 @@ __global__ void __launch_bounds__(256, 2) rs_mc_adamw_kernel(const TIn* mc_grad,
         load8(a.m + j, mm);
         load8(a.v + j, vv);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) adamw_one(pp[e], mm[e], vv[e], acc[e] * scale, a);
+        for (int e = 0; e < 8; ++e) adamw_update(pp[e], mm[e], vv[e], acc[e] * scale, a.step);
         store8(a.p + j, pp);
         store8(a.m + j, mm);
         store8(a.v + j, vv);
@@ -693,16 +686,15 @@ static bool adamw_ptrs_ok(const float* p, const float* m, const float* v, const 
 MFSDP_API int mfsdp_rs_pull_adamw(const unsigned long long* grad_ptrs_host, int world, int rank,
                                   const long long* global_off, const long long* local_off, const long long* len,
                                   int nseg, long long max_len, int in_is_bf16, float scale, float* p, float* m,
-                                  float* v, void* p_lp, float lr, float beta1, float beta2, float eps,
-                                  float weight_decay, int step, const int* status, cudaStream_t st) {
+                                  float* v, void* p_lp, double lr, double beta1, double beta2, double eps,
+                                  double weight_decay, int step, const int* status, cudaStream_t st) {
   if (nseg <= 0) return 0;
   if (world <= 0 || world > kMaxPeers || step < 1) return -2;
   if (!adamw_ptrs_ok(p, m, v, p_lp)) return -2;
   PeerPtrs pp{};
   for (int i = 0; i < world; ++i) pp.p[i] = reinterpret_cast<const void*>(grad_ptrs_host[i]);
   ReduceTable tab{global_off, local_off, len};
-  AdamWArgs a{p, m, v, (__nv_bfloat16*)p_lp, lr, beta1, beta2, eps, weight_decay,
-              1.f - powf(beta1, (float)step), sqrtf(1.f - powf(beta2, (float)step))};
+  const AdamWArgs a{p, m, v, (__nv_bfloat16*)p_lp, adamw_step(lr, beta1, beta2, eps, weight_decay, step, 1.0)};
   const dim3 grid = seg_grid(max_len, 8, nseg);
 #define MFSDP_RA(TI)                                                                                              \
   do {                                                                                                            \
@@ -778,13 +770,12 @@ MFSDP_API int mfsdp_rs_mc_reduce(const void* mc_grad, void* out, const long long
 
 MFSDP_API int mfsdp_rs_mc_adamw(const void* mc_grad, const long long* global_off, const long long* local_off,
                                 const long long* len, int nseg, long long max_len, int in_is_bf16, float scale,
-                                float* p, float* m, float* v, void* p_lp, float lr, float beta1, float beta2, float eps,
-                                float weight_decay, int step, const int* status, cudaStream_t st) {
+                                float* p, float* m, float* v, void* p_lp, double lr, double beta1, double beta2,
+                                double eps, double weight_decay, int step, const int* status, cudaStream_t st) {
   if (nseg <= 0) return 0;
   if (step < 1 || ((uintptr_t)mc_grad % 16) || !adamw_ptrs_ok(p, m, v, p_lp)) return -2;
   ReduceTable tab{global_off, local_off, len};
-  AdamWArgs a{p, m, v, (__nv_bfloat16*)p_lp, lr, beta1, beta2, eps, weight_decay,
-              1.f - powf(beta1, (float)step), sqrtf(1.f - powf(beta2, (float)step))};
+  const AdamWArgs a{p, m, v, (__nv_bfloat16*)p_lp, adamw_step(lr, beta1, beta2, eps, weight_decay, step, 1.0)};
   const dim3 grid = nvls_grid(max_len / 8, nseg);
   if (in_is_bf16) rs_mc_adamw_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)mc_grad, tab, nseg, scale, a, status);
   else rs_mc_adamw_kernel<float><<<grid, 256, 0, st>>>((const float*)mc_grad, tab, nseg, scale, a, status);

@@ -64,11 +64,11 @@ _lib.register_signatures({
     "mfsdp_rs_pull_reduce": [C.POINTER(_u64), _i32, _i32, _vp, _vp, _vp, _vp, _i32, _i64, _i32, _i32, _i32,
                              C.c_float, _vp, _vp],
     "mfsdp_rs_pull_adamw": [C.POINTER(_u64), _i32, _i32, _vp, _vp, _vp, _i32, _i64, _i32, C.c_float, _vp, _vp, _vp,
-                            _vp, C.c_float, C.c_float, C.c_float, C.c_float, C.c_float, _i32, _vp, _vp],
+                            _vp, *[C.c_double] * 5, _i32, _vp, _vp],
     "mfsdp_ag_push_mc": [_vp, _vp, _vp, _vp, _vp, _i32, _i64, _vp, _vp],
     "mfsdp_rs_mc_reduce": [_vp, _vp, _vp, _vp, _vp, _i32, _i64, _i32, _i32, _i32, C.c_float, _vp, _vp],
-    "mfsdp_rs_mc_adamw": [_vp, _vp, _vp, _vp, _i32, _i64, _i32, C.c_float, _vp, _vp, _vp, _vp, C.c_float, C.c_float,
-                          C.c_float, C.c_float, C.c_float, _i32, _vp, _vp],
+    "mfsdp_rs_mc_adamw": [_vp, _vp, _vp, _vp, _i32, _i64, _i32, C.c_float, _vp, _vp, _vp, _vp, *[C.c_double] * 5,
+                          _i32, _vp, _vp],
     "mfsdp_ar_mc": [_vp, _i64, _i32, _i32, _i32, C.c_float, _vp, _vp],
 })
 

@@ -559,3 +559,56 @@ def test_adamw_records_the_low_precision_copy_for_autograd():
     version = shard._version
     opt.step()
     assert torch.equal(shard[64:], p.detach().bfloat16()) and shard._version > version
+
+
+def _adamw_64(p, m, v, g, step, lr, beta1, beta2, eps, weight_decay):
+    m.mul_(beta1).add_(g, alpha=1 - beta1)
+    v.mul_(beta2).addcmul_(g, g, value=1 - beta2)
+    p.mul_(1 - lr * weight_decay).sub_(lr / (1 - beta1 ** step) * m / ((v / (1 - beta2 ** step)).sqrt() + eps))
+
+
+@pytest.mark.parametrize("route", ["outside units", "flat", "reduction"])
+@pytest.mark.parametrize("betas", [(0.9, 0.95), (0.9, 0.999), (0.0, 0.99999)])
+@pytest.mark.parametrize("first", [1, 1000])
+def test_adamw_constants_and_rounding(K, route, betas, first):
+    """Three steps from step ``first`` against 64 bits, on each way into the update.  Moments: a handful of fp32 roundings
+    a step (the smallest ones, below the normal range, to two units of their spacing); the distance covered by the
+    parameter: the same, plus 2.5 * 2^-24 of the parameter itself per step (decay factor, its product, the sum)."""
+    import ctypes as C
+
+    from matrix_fsdp_b200.ops import lib
+    from matrix_fsdp_b200.optim.flat import FlatShardedAdamW
+    from matrix_fsdp_b200.parallel import peer  # noqa: F401  (its entries' signatures)
+
+    torch.manual_seed(first)
+    n, hp = 4099, dict(lr=1e-3, eps=1e-8, weight_decay=0.1)
+    p0 = torch.randn(n, device="cuda")
+    m0, v0 = 1e-3 * torch.randn(n, device="cuda"), 1e-6 * torch.rand(n, device="cuda")
+    if first == 1:
+        m0.zero_(), v0.zero_()
+    p, m, v = torch.nn.Parameter(p0.clone()), m0.clone(), v0.clone()
+    want = [t.double() for t in (p0, m0, v0)]
+    opt = FlatShardedAdamW([p], betas=betas, **hp)
+    opt.state[p] = dict(step=torch.tensor(float(first - 1)), exp_avg=m, exp_avg_sq=v)
+    seg = torch.tensor([0, 0, n], device="cuda")
+    for step in range(first, first + 3):
+        p.grad = 1e-3 * torch.randn(n, device="cuda")
+        p.grad[:32] = 1e-20
+        if route == "outside units":
+            opt.step()
+        elif route == "flat":
+            K.adamw_flat_(p.data, m, v, p.grad, beta1=betas[0], beta2=betas[1], step=step, **hp)
+        else:
+            # one rank reducing its own gradient: no peer to wait for
+            status = K.status_word()
+            rc = lib.load(required=True).mfsdp_rs_pull_adamw(
+                (C.c_ulonglong * 1)(p.grad.data_ptr()), 1, 0, seg.data_ptr(), seg[1:].data_ptr(), seg[2:].data_ptr(), 1, n, 0,
+                1.0, p.data_ptr(), m.data_ptr(), v.data_ptr(), None, hp["lr"], *betas, hp["eps"], hp["weight_decay"], step,
+                status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+            assert rc == 0
+        _adamw_64(*want, p.grad.double(), step, beta1=betas[0], beta2=betas[1], **hp)
+    K.check_status()
+    assert ((m.double() - want[1]).abs() <= 1e-6 * want[1].abs() + 3 * 2 ** -24 * 3e-3).all()
+    assert ((v.double() - want[2]).abs() <= 1e-6 * want[2] + 6 * 2 ** -149).all()
+    moved = (want[0] - p0.double()).abs()
+    assert ((p.detach().double() - want[0]).abs() <= 2e-6 * moved + 4 * 2 ** -23 * p0.double().abs().clamp_min(2 ** -8)).all()
