@@ -38,6 +38,12 @@ def _stream() -> int:
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
+def on_current_device(t: torch.Tensor) -> bool:
+    """Launches go to the current device's stream.  Torch operations switch to their tensors' device; a caller that has
+    both ways takes them for a tensor that lives elsewhere."""
+    return t.is_cuda and t.get_device() == torch._C._cuda_getDevice()
+
+
 def _launch_context(device: torch.device) -> tuple[int, int]:
     """Address of the device's status word and its number of SMs."""
     ctx = _CONTEXT.get(device)

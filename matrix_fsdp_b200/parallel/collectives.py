@@ -177,7 +177,7 @@ def _copy_segment(dst: torch.Tensor, src: torch.Tensor) -> None:
             and src.is_contiguous() and dst.is_contiguous():
         from ..ops import kernels, lib
 
-        if lib.available() and not lib.disabled_by_env():
+        if lib.available() and not lib.disabled_by_env() and kernels.on_current_device(src):
             kernels.cast_bf16_f32(src, dst)
             return
     dst.copy_(src)

@@ -80,7 +80,7 @@ def clip_grad_norm_(module_or_units, max_norm: float, norm_type: float = 2.0,
             return None
         from ..ops import kernels, lib
 
-        return kernels if lib.available() and not lib.disabled_by_env() else None
+        return kernels if lib.available() and not lib.disabled_by_env() and kernels.on_current_device(g) else None
 
     def power_sum(g):
         g = g.detach()

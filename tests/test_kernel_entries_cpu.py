@@ -82,3 +82,44 @@ def test_a_scaled_loss_is_not_walked_twice_over_one_graph(library):
     assert (grad.float() - want).abs().max() <= 2 ** -7 * want.abs().max()      # two bf16 roundings
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         torch.autograd.grad(loss, logits)
+
+
+class _OnDevice(torch.Tensor):
+    """A CPU tensor that says it lives on a CUDA device."""
+
+    is_cuda = True
+
+    def get_device(self):
+        return 1
+
+
+@pytest.mark.parametrize("current", [0, 1])
+def test_kernels_take_tensors_of_the_current_device_only(library, monkeypatch, current):
+    """A launch goes to the current device; tensors of another one keep the torch operations, which switch to it."""
+    from matrix_fsdp_b200.ops import lib
+    from matrix_fsdp_b200.optim import flat
+    from matrix_fsdp_b200.parallel import collectives
+    from matrix_fsdp_b200.utils import training
+
+    launched = []
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: current, raising=False)
+    monkeypatch.setattr(lib, "available", lambda: True)
+    monkeypatch.setattr(flat, "_native", lambda device: True)
+    monkeypatch.setattr(K, "sumsq", lambda x: launched.append("sumsq") or x.double().pow(2).sum().float())
+    monkeypatch.setattr(K, "scale_", lambda x, s: launched.append("scale") or x.mul_(s))
+    monkeypatch.setattr(K, "cast_bf16_f32", lambda s, d: launched.append("cast") or d.copy_(s))
+
+    g = torch.randn(32).as_subclass(_OnDevice)
+    before = g.clone()
+    training.clip_grad_norm_([], 1.0, extra_grads=[g])
+    assert torch.allclose(g.norm(), torch.ones(()), atol=1e-4) and not torch.equal(g, before)
+
+    src, dst = torch.randn(16).bfloat16().as_subclass(_OnDevice), torch.zeros(16).as_subclass(_OnDevice)
+    collectives._copy_segment(dst, src)
+    assert torch.equal(dst, src.float())
+
+    p, g = torch.randn(16).as_subclass(_OnDevice), torch.randn(16).as_subclass(_OnDevice)
+    p.grad = g
+    state = dict(exp_avg=torch.zeros(16).as_subclass(_OnDevice), exp_avg_sq=torch.zeros(16).as_subclass(_OnDevice))
+    assert flat.FlatShardedAdamW._one_kernel(p, state) == (current == 1)
+    assert launched == (["sumsq", "scale", "cast"] if current == 1 else [])
