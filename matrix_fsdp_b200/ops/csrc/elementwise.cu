@@ -981,7 +981,8 @@ MFSDP_API int mfsdp_rmsnorm_bwd(const void* dy, const void* x, const void* w, co
                                 const void* dres, void* dx, float* dw_acc, void* dw,
                                 int accumulate_dw, long long rows, int H, cudaStream_t st) {
   if (H % 8 || H > 8 * 4 * 256) return -2;
-  if (rows <= 0) return -2;
+  if (rows <= 0)                              // no rows: the weight gradient is zero
+    return dw && !accumulate_dw ? (int)cudaMemsetAsync(dw, 0, (size_t)H * sizeof(__nv_bfloat16), st) : 0;
   const int grid = launch_rmsnorm_bwd((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
                                       (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw_acc, rows, H, kRmsBwdCtas, st);
   if (dw) launch_pdl(colsum_f32_to_bf16_kernel, dim3((H + 31) / 32), dim3(32, 8), 0, st, dw_acc, (__nv_bfloat16*)dw, grid, H, accumulate_dw);

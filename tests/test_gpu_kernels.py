@@ -612,3 +612,20 @@ def test_adamw_constants_and_rounding(K, route, betas, first):
     assert ((v.double() - want[2]).abs() <= 1e-6 * want[2] + 6 * 2 ** -149).all()
     moved = (want[0] - p0.double()).abs()
     assert ((p.detach().double() - want[0]).abs() <= 2e-6 * moved + 4 * 2 ** -23 * p0.double().abs().clamp_min(2 ** -8)).all()
+
+
+def test_rmsnorm_of_no_rows(K):
+    """An empty batch goes through both directions; it adds nothing to the weight's gradient."""
+    from matrix_fsdp_b200.ops import functional as OF
+
+    x, w = torch.empty(0, 264, device="cuda", dtype=torch.bfloat16), _rand(264)
+    y, rstd = K.rmsnorm_fwd(x, w, 1e-5)
+    assert y.shape == x.shape and rstd.shape == (0,)
+    dx, dw = K.rmsnorm_bwd(y, x, w, rstd)
+    assert dx.shape == x.shape and torch.equal(dw, torch.zeros_like(w))
+    old = w.clone()
+    K.rmsnorm_bwd(y, x, w, rstd, dw_out=old, accumulate_dw=True)
+    assert torch.equal(old, w)
+    x.requires_grad_(True), w.requires_grad_(True)
+    gx, gw = torch.autograd.grad(OF.rms_norm(x, w).sum(), (x, w))
+    assert gx.shape == x.shape and torch.equal(gw, torch.zeros_like(w))
