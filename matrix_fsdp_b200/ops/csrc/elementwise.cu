@@ -12,55 +12,6 @@
 namespace mfsdp {
 
 // ============================================================== RMSNorm
-// One CTA per row; H <= 8 * 8 * blockDim (each thread keeps up to 8 vectors of 8 bf16).
-template <int VPT>
-__global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
-                                   const __nv_bfloat16* __restrict__ w,
-                                   __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out,
-                                   int H, float eps) {
-  __shared__ float red[32];
-  const long long row = blockIdx.x;
-  const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
-  const uint4* wr = reinterpret_cast<const uint4*>(w);
-  uint4* yr = reinterpret_cast<uint4*>(y + row * H);
-  const int nvec = H >> 3;
-  uint4 xv[VPT];
-  float ss = 0.f;
-#pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int v = threadIdx.x + i * blockDim.x;
-    if (v < nvec) {
-      xv[i] = xr[v];
-      const uint32_t u[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = unpack_bf16x2(u[e]);
-        ss += f.x * f.x + f.y * f.y;
-      }
-    }
-  }
-  ss = block_sum(ss, red);
-  const float rstd = rsqrtf(ss / (float)H + eps);
-  if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
-#pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int v = threadIdx.x + i * blockDim.x;
-    if (v < nvec) {
-      const uint4 wv = wr[v];
-      const uint32_t u[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w};
-      const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
-      uint32_t o[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = unpack_bf16x2(u[e]);
-        const float2 g = unpack_bf16x2(ww[e]);
-        o[e] = pack_bf16x2(f.x * rstd * g.x, f.y * rstd * g.y);
-      }
-      yr[v] = make_uint4(o[0], o[1], o[2], o[3]);
-    }
-  }
-}
-
 // WPR warps per row, 8 / WPR rows per CTA, VPL vectors of 8 per lane: a row's sum needs shuffles and at most one
 // barrier, and the rows of a CTA wait for nobody else's memory.  One CTA per row -> this: 4096 rows of 2048 14.3 -> 12.3
 // us, 16384 rows of 4096 54.1 -> 51.2 us (5.2 TB/s), 515 rows of 1024 8.1 -> 7.1 us.
@@ -941,19 +892,16 @@ using namespace mfsdp;
 
 MFSDP_API int mfsdp_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long long rows,
                                 int H, float eps, cudaStream_t st) {
-  if (H % 8 || H > 8 * 8 * 1024) return -2;
+  if (H % 8 || H > 8 * 8 * 256) return -2;    // 16384 columns: a CTA's 256 threads hold a row in 8 vectors each
   if (rows <= 0) return 0;
   const int nvec = H / 8;
   auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w; auto Y = (__nv_bfloat16*)y;
-  // up to 16384 columns a row's warps hold it in 8 vectors per lane; beyond that one CTA takes a row
   auto rows_kernel = nvec <= 64 ? rmsnorm_fwd_rows_kernel<2, 1> : nvec <= 128 ? rmsnorm_fwd_rows_kernel<4, 1> :
                      nvec <= 256 ? rmsnorm_fwd_rows_kernel<8, 1> : nvec <= 512 ? rmsnorm_fwd_rows_kernel<8, 2> :
                      nvec <= 1024 ? rmsnorm_fwd_rows_kernel<8, 4> : rmsnorm_fwd_rows_kernel<8, 8>;
   const int rpc = nvec <= 256 ? 8 : nvec <= 512 ? 4 : nvec <= 1024 ? 2 : 1;
-  if (nvec <= 2048) return launch_pdl(rows_kernel, dim3((unsigned)((rows + rpc - 1) / rpc)), dim3(256), 0, st, X, W, Y, rstd, rows, H, eps);
-  if (nvec <= 8 * 1024) rmsnorm_fwd_kernel<8><<<(unsigned)rows, 1024, 0, st>>>(X, W, Y, rstd, H, eps);
-  else return -2;
-  return (int)cudaGetLastError();
+  return launch_pdl(rows_kernel, dim3((unsigned)((rows + rpc - 1) / rpc)), dim3(256), 0, st, X, W, Y, rstd,
+                    rows, H, eps);
 }
 
 // Upper bound of the backward kernel's CTAs (= rows of the dw scratch matrix).

@@ -629,3 +629,21 @@ def test_rmsnorm_of_no_rows(K):
     x.requires_grad_(True), w.requires_grad_(True)
     gx, gw = torch.autograd.grad(OF.rms_norm(x, w).sum(), (x, w))
     assert gx.shape == x.shape and torch.equal(gw, torch.zeros_like(w))
+
+
+@pytest.mark.parametrize("rows", [1, 3, 150])
+@pytest.mark.parametrize("H", [8200, 12296, 16384])
+def test_rmsnorm_forward_of_the_widest_rows(K, rows, H):
+    """Eight warps per row, up to the last width that a CTA's registers hold; wider rows are refused."""
+    torch.manual_seed(rows + H)
+    x, w = _rand(rows, H), (1 + 0.1 * torch.randn(H, device="cuda")).bfloat16()
+    y, rstd = K.rmsnorm_fwd(x, w, 1e-5)
+    want = torch.rsqrt(x.double().pow(2).mean(-1) + 1e-5)
+    assert torch.allclose(rstd.double(), want, rtol=1e-5)
+    assert _rel_err(y, x.double() * want[:, None] * w.double()) < 2 ** -8
+
+
+def test_rmsnorm_refuses_rows_wider_than_a_block_holds(K):
+    x, w = _rand(2, 16392), _rand(16392)
+    with pytest.raises(RuntimeError):
+        K.rmsnorm_fwd(x, w, 1e-5)
