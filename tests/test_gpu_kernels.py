@@ -647,3 +647,71 @@ def test_rmsnorm_refuses_rows_wider_than_a_block_holds(K):
     x, w = _rand(2, 16392), _rand(16392)
     with pytest.raises(RuntimeError):
         K.rmsnorm_fwd(x, w, 1e-5)
+
+
+@pytest.mark.parametrize("where", ["current stream", "second stream", "captured"])
+def test_dependent_launches_keep_stream_order(K, where):
+    """Kernels that may start before their predecessor has ended wait for it before they touch memory: a chain whose
+    buffers are freed behind each launch (the next kernel writes into what its predecessor still reads, if it is early)
+    gives the bits of the same chain with a synchronisation after every launch."""
+    from matrix_fsdp_b200.ops import attention as A
+
+    torch.manual_seed(0)
+    B, S, nH, F = 2, 200, 2, 328
+    H, T, V = nH * 128, B * S, 1000
+    x, dy = torch.empty(T, H, device="cuda", dtype=torch.bfloat16), _rand(T, H)
+    w = (1 + 0.1 * torch.randn(H, device="cuda")).bfloat16()
+    qkv_w, o_w, gu_w, d_w, head = (_rand(n, k, scale=k ** -0.5) for n, k in ((3 * H, H), (H, H), (2 * F, H), (H, F), (V, H)))
+    angles = torch.randn(S, 64, device="cuda")
+    cos, sin = angles.cos(), angles.sin()
+    target = torch.randint(0, V, (T,), device="cuda")
+
+    def chain(after=lambda: None):
+        def run(fn, *args, **kw):
+            out = fn(*args, **kw)
+            after()
+            return out
+
+        y, rstd = run(K.rmsnorm_fwd, x, w, 1e-5)
+        qkv = run(K.gemm, y, qkv_w)
+        del y
+        run(K.rope_, qkv, cos, sin, S, 0, 2 * nH, 128)
+        att, lse = run(A.attention_fwd, qkv, B, S, nH, 128)
+        h = run(K.gemm, att, o_w, cin=x, beta=1.0)
+        gu = run(K.gemm, h, gu_w)
+        act = run(K.swiglu_fwd, gu)
+        dgu = run(K.swiglu_bwd, act, gu)
+        del gu
+        out = run(K.gemm, act, d_w, cin=h, beta=1.0)
+        del act
+        logits = run(K.gemm, out, head)
+        loss = run(K.cross_entropy_, logits, target, 1.0 / T)
+        dout = run(K.gemm, logits, head, b_mn_major=True)
+        del logits
+        dqkv = run(A.attention_bwd, dout, qkv, att, lse, B, S, nH, 128)
+        del qkv, att, lse
+        dx, dw = run(K.rmsnorm_bwd, dy, x, w, rstd, dres=dout)
+        return loss, dgu, out, dqkv, dx, dw
+
+    stream = torch.cuda.Stream() if where != "current stream" else torch.cuda.current_stream()
+    if where == "captured":
+        x.copy_(_rand(T, H))
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            chain()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            got = chain()
+    for _ in range(10):
+        x.copy_(_rand(T, H))
+        want = chain(torch.cuda.synchronize)
+        if where == "captured":
+            graph.replay()
+        else:
+            stream.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(stream):
+                got = chain()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    K.check_status()
