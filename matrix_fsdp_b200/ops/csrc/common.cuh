@@ -476,7 +476,9 @@ __device__ __forceinline__ float ieee_sqrt(float a) { float d; asm("sqrt.rn.f32 
 
 __device__ __forceinline__ void adamw_update(float& p, float& m, float& v, float g, const AdamWStep& a) {
   g = ieee_mul(g, a.grad_scale);
-  m = ieee_fma(a.beta1, m, ieee_mul(a.one_minus_beta1, g));
+  // between m and g from the nearer end, as torch's lerp: one rounded constant instead of two that do not add up to one
+  const float d = ieee_add(g, -m);
+  m = a.one_minus_beta1 < 0.5f ? ieee_fma(a.one_minus_beta1, d, m) : ieee_fma(-a.beta1, d, g);
   v = ieee_fma(a.beta2, v, ieee_mul(ieee_mul(a.one_minus_beta2, g), g));
   const float denom = ieee_add(ieee_div(ieee_sqrt(v), a.bias2_sqrt), a.eps);
   p = ieee_fma(-a.step_size, ieee_div(m, denom), ieee_mul(p, a.keep));
