@@ -779,21 +779,25 @@ __global__ void __launch_bounds__(256) embed_place_kernel(const long long* __res
 // Up to this many positions of one id are ordered by counting the smaller ones (n^2 comparisons by one block); a more
 // frequent id (padding) has its positions collected again, in order, from the ids themselves.
 constexpr int kEmbedSortMax = 256;
+// Rows of a frequent id in flight.  One block adds them all up, in order, so what counts is how many it has under way:
+// as asynchronous copies they cost no registers, and 24 KB leave the SM its eight blocks.
+constexpr int kEmbedRing = 6;
 
-__global__ void __launch_bounds__(256) embed_sum_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy,
-                                                        __nv_bfloat16* __restrict__ dw, long long lddw, int H,
-                                                        const long long* __restrict__ ids, int T,
-                                                        const int* __restrict__ count, const int* __restrict__ cursor,
-                                                        const int* __restrict__ place, int* __restrict__ order_buf,
-                                                        int accumulate) {
+__global__ void __launch_bounds__(256, 8) embed_sum_kernel(const __nv_bfloat16* __restrict__ dy, long long lddy,
+                                                           __nv_bfloat16* __restrict__ dw, long long lddw, int H,
+                                                           const long long* __restrict__ ids, int T,
+                                                           const int* __restrict__ count, const int* __restrict__ cursor,
+                                                           const int* __restrict__ place, int* __restrict__ order_buf,
+                                                           int accumulate) {
   __shared__ int list[kEmbedSortMax];
   __shared__ int sorted[kEmbedSortMax];
   __shared__ int warp_tot[8];
+  __shared__ uint4 ring[kEmbedRing][256];
   const int v = blockIdx.x;
   const int n = count[v];
   if (n == 0 && accumulate) return;
   const int first = cursor[v] - n;
-  const int* order = sorted;
+  __nv_bfloat16* out = dw + (long long)v * lddw;
   if (n <= kEmbedSortMax) {
     if (threadIdx.x < n) list[threadIdx.x] = place[first + threadIdx.x];
     __syncthreads();
@@ -804,41 +808,73 @@ __global__ void __launch_bounds__(256) embed_sum_kernel(const __nv_bfloat16* __r
       sorted[rank] = mine;
     }
     __syncthreads();
-  } else {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int run = first;
-    for (int base = 0; base < T; base += 256) {
-      const int t = base + threadIdx.x;
-      const bool hit = t < T && ids[t] == v;
-      const unsigned m = __ballot_sync(0xffffffffu, hit);
-      if (lane == 0) warp_tot[warp] = __popc(m);
-      __syncthreads();
-      int before = 0, total = 0;
+    for (int c = threadIdx.x * 8; c < H; c += 256 * 8) {
+      float acc[8];
 #pragma unroll
-      for (int w = 0; w < 8; ++w) {
-        if (w < warp) before += warp_tot[w];
-        total += warp_tot[w];
+      for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+      if (accumulate) load8(out + c, acc);
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) {
+        float f[8];
+        load8(dy + (long long)sorted[j] * lddy + c, f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += f[e];
       }
-      if (hit) order_buf[run + before + __popc(m & ((1u << lane) - 1u))] = t;
-      run += total;
-      __syncthreads();
+      *reinterpret_cast<uint4*>(out + c) = pack8(acc);
     }
-    order = order_buf + first;                        // written by this block, read after the barrier
+    return;
   }
-  __nv_bfloat16* out = dw + (long long)v * lddw;
-  for (int c = threadIdx.x * 8; c < H; c += 256 * 8) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int run = first;
+  for (int base = 0; base < T; base += 256) {
+    const int t = base + threadIdx.x;
+    const bool hit = t < T && ids[t] == v;
+    const unsigned m = __ballot_sync(0xffffffffu, hit);
+    if (lane == 0) warp_tot[warp] = __popc(m);
+    __syncthreads();
+    int before = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      if (w < warp) before += warp_tot[w];
+      total += warp_tot[w];
+    }
+    if (hit) order_buf[run + before + __popc(m & ((1u << lane) - 1u))] = t;
+    run += total;
+    __syncthreads();
+  }
+  for (int c0 = 0; c0 < H; c0 += 256 * 8) {
+    const int c = c0 + threadIdx.x * 8;
+    const bool mine = c < H;                            // every thread takes part in the barriers
     float acc[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-    if (accumulate) load8(out + c, acc);
-#pragma unroll 4
-    for (int j = 0; j < n; ++j) {
-      float f[8];
-      load8(dy + (long long)order[j] * lddy + c, f);
+    if (mine && accumulate) load8(out + c, acc);
+    for (int base = 0; base < n; base += kEmbedSortMax) {
+      const int m = min(n - base, kEmbedSortMax);
+      __syncthreads();                                  // order_buf is written, the last part of the list used up
+      if (threadIdx.x < m) sorted[threadIdx.x] = order_buf[first + base + threadIdx.x];
+      __syncthreads();
+      if (mine) {
+        auto fetch = [&](int j, int slot) {             // a thread reads only what it copied itself
+          if (j < m) cp_async16(smem_u32(&ring[slot][threadIdx.x]), dy + (long long)sorted[j] * lddy + c);
+          cp_async_commit();
+        };
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] += f[e];
+        for (int j = 0; j < kEmbedRing; ++j) fetch(j, j);
+        int slot = 0;
+        for (int j = 0; j < m; ++j) {
+          cp_async_wait<kEmbedRing - 1>();
+          float f[8];
+          load8(reinterpret_cast<const __nv_bfloat16*>(&ring[slot][threadIdx.x]), f);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc[e] += f[e];
+          fetch(j + kEmbedRing, slot);
+          slot = slot + 1 == kEmbedRing ? 0 : slot + 1;
+        }
+        cp_async_wait<0>();
+      }
     }
-    *reinterpret_cast<uint4*>(out + c) = pack8(acc);
+    if (mine) *reinterpret_cast<uint4*>(out + c) = pack8(acc);
   }
 }
 

@@ -715,3 +715,24 @@ def test_dependent_launches_keep_stream_order(K, where):
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip(got, want))
     K.check_status()
+
+
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("n,H", [(257, 8), (261, 2056), (262, 72), (512, 2048), (513, 4104)])
+def test_embedding_backward_of_a_frequent_id(K, n, H, accumulate):
+    """More positions of one id than a block sorts: whole and partial lists of 256, remainders of the copies in flight,
+    column ranges that leave threads idle.  The fp32 sum in the order of the positions, bit for bit."""
+    torch.manual_seed(n)
+    ids = torch.full((2 * n,), 3, device="cuda")
+    ids[1::2] = torch.randint(4, 40, (n,), device="cuda")
+    dy, old = _rand(2 * n, H), _rand(41, H)
+    out = old.clone()
+    K.embedding_bwd(dy, ids, out, accumulate=accumulate)
+    want = old[3].float() if accumulate else torch.zeros(H, device="cuda")
+    for row in dy[0::2].float():
+        want = want + row
+    assert torch.equal(out[3], want.bfloat16())
+    total = torch.zeros(41, H, dtype=torch.float64, device="cuda").index_add_(0, ids, dy.double())
+    if accumulate:
+        total += old.double()
+    assert _rel_err(out, total) < 2 ** -8
