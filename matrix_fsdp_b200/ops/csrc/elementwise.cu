@@ -13,8 +13,8 @@ namespace mfsdp {
 
 // ============================================================== RMSNorm
 // WPR warps per row, 8 / WPR rows per CTA, VPL vectors of 8 per lane: a row's sum needs shuffles and at most one
-// barrier, and the rows of a CTA wait for nobody else's memory.  One CTA per row -> this: 4096 rows of 2048 14.3 -> 12.3
-// us, 16384 rows of 4096 54.1 -> 51.2 us (5.2 TB/s), 515 rows of 1024 8.1 -> 7.1 us.
+// barrier, and the rows of a CTA wait for nobody else's memory.  Bound by memory.  One CTA per row -> this: 4096 rows of
+// 2048 6.8 -> 5.0 us, 16384 rows of 4096 47.8 -> 41.6 us (6.4 TB/s), of 5120 60.6 -> 54.8, of 12288 174 -> 143.
 template <int VPL, int WPR>
 __global__ void __launch_bounds__(256)
 rmsnorm_fwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
@@ -77,11 +77,12 @@ rmsnorm_fwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
 // dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres);  dw += sum_rows dy * xhat.
 // Persistent over rows, WPR warps per row and 8 / WPR rows per CTA at a time: a row's dot product needs shuffles and, for
 // WPR > 1, a barrier of its own warps only.  The weight gradient stays in registers until the end, when the warps of a
-// CTA add theirs up in shared memory, in a fixed order, into one partial row per CTA.  Bound by memory.  One CTA per two
-// or four rows, barriers of the whole block -> this, residual included: 4096 rows of 2048 35.8 -> 27.6 us, 16384 rows of
-// 4096 148 -> 116 us (4.6 TB/s), 4096 rows of 8192 134 -> 77 us.
-template <int VPL, int WPR>
-__global__ void __launch_bounds__(256, 1)
+// CTA add theirs up in shared memory, in a fixed order, into one partial row per CTA.  Bound by memory.  RES: with the
+// residual's gradient dres, in a kernel of its own because its registers decide how many CTAs fit.  One CTA per two
+// or four rows, barriers of the whole block -> this, residual included: 4096 rows of 2048 18.6 -> 11.5 us, 16384 rows of
+// 4096 140 -> 105 us (5.1 TB/s), 4096 rows of 8192 126 -> 66 us; without: 15.0 -> 10.6, 82.9 -> 77.5, 69 -> 57.
+template <int VPL, int WPR, int CTAS, bool RES>
+__global__ void __launch_bounds__(256, CTAS)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
@@ -112,7 +113,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
       const bool in = v < nvec;
       xv[i] = in ? reinterpret_cast<const uint4*>(x + row * H)[v] : make_uint4(0, 0, 0, 0);
       dv[i] = in ? reinterpret_cast<const uint4*>(dy + row * H)[v] : make_uint4(0, 0, 0, 0);
-      rv[i] = in && dres ? reinterpret_cast<const uint4*>(dres + row * H)[v] : make_uint4(0, 0, 0, 0);
+      if (RES) rv[i] = in ? reinterpret_cast<const uint4*>(dres + row * H)[v] : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
@@ -151,7 +152,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
           o[2 * e] = rstd * (df.x * wf.x - xf.x * rstd * mean_dot);
           o[2 * e + 1] = rstd * (df.y * wf.y - xf.y * rstd * mean_dot);
         }
-        if (dres) {
+        if (RES) {
           const uint32_t ru[4] = {rv[i].x, rv[i].y, rv[i].z, rv[i].w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
@@ -935,31 +936,68 @@ MFSDP_API int mfsdp_rmsnorm_fwd(const void* x, const void* w, void* y, float* rs
   if (rows <= 0) return 0;
   const int nvec = H / 8;
   auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w; auto Y = (__nv_bfloat16*)y;
-  auto rows_kernel = nvec <= 64 ? rmsnorm_fwd_rows_kernel<2, 1> : nvec <= 128 ? rmsnorm_fwd_rows_kernel<4, 1> :
-                     nvec <= 256 ? rmsnorm_fwd_rows_kernel<8, 1> : nvec <= 512 ? rmsnorm_fwd_rows_kernel<8, 2> :
-                     nvec <= 1024 ? rmsnorm_fwd_rows_kernel<8, 4> : rmsnorm_fwd_rows_kernel<8, 8>;
-  const int rpc = nvec <= 256 ? 8 : nvec <= 512 ? 4 : nvec <= 1024 ? 2 : 1;
-  return launch_pdl(rows_kernel, dim3((unsigned)((rows + rpc - 1) / rpc)), dim3(256), 0, st, X, W, Y, rstd,
-                    rows, H, eps);
+  // As few warps per row as hold it in four vectors per lane, eight beyond 8192 columns, and no more vectors per lane than
+  // that takes: what a lane does not use still costs registers, and with them rows in flight (16384 rows of 5120 columns:
+  // 54.8 us with 8 x 3 vectors, 70.3 with 4 x 8; of 4096: 41.6 with 4 x 4, 45.1 with 2 x 8).
+  const int wpr = nvec <= 128 ? 1 : nvec <= 256 ? 2 : nvec <= 512 ? 4 : 8;
+  const int rpc = 8 / wpr, vpl = (nvec + 32 * wpr - 1) / (32 * wpr);
+  const dim3 grid((unsigned)((rows + rpc - 1) / rpc));
+#define MFSDP_RMS(VPL, WPR) \
+  if (vpl <= VPL && wpr == WPR) return launch_pdl(rmsnorm_fwd_rows_kernel<VPL, WPR>, grid, dim3(256), 0, st, X, W, Y, rstd, rows, H, eps)
+  MFSDP_RMS(1, 1); MFSDP_RMS(2, 1); MFSDP_RMS(3, 1); MFSDP_RMS(4, 1);
+  MFSDP_RMS(3, 2); MFSDP_RMS(4, 2);
+  MFSDP_RMS(3, 4); MFSDP_RMS(4, 4);
+  MFSDP_RMS(3, 8); MFSDP_RMS(4, 8); MFSDP_RMS(5, 8); MFSDP_RMS(6, 8); MFSDP_RMS(7, 8); MFSDP_RMS(8, 8);
+#undef MFSDP_RMS
+  return -2;
 }
 
-// Upper bound of the backward kernel's CTAs (= rows of the dw scratch matrix).
-constexpr int kRmsBwdCtas = 148;              // resident at once
+// Upper bound of the backward kernel's CTAs (= rows of the dw scratch matrix): at most three are resident per SM.
+constexpr int kRmsBwdCtas = 3 * 148;
 MFSDP_API int mfsdp_rmsnorm_bwd_scratch_rows(long long rows) { return (int)(rows < kRmsBwdCtas ? (rows < 1 ? 1 : rows) : kRmsBwdCtas); }
 
 // Launches the backward kernel on at most `cap` CTAs, each with the same number of trips (up to rounding); returns the
 // number of partial rows that it writes to dw_acc.
+template <int VPL, int WPR, int CTAS, bool RES>
+static int launch_rmsnorm_bwd_as(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w, const float* rstd,
+                                 const __nv_bfloat16* dres, __nv_bfloat16* dx, float* dw_acc, long long rows, int H, int cap,
+                                 cudaStream_t st) {
+  constexpr int RPC = 8 / WPR;
+  const long long groups = (rows + RPC - 1) / RPC, trips = (groups + cap - 1) / cap;
+  const int grid = (int)((groups + trips - 1) / trips);
+  launch_pdl(rmsnorm_bwd_kernel<VPL, WPR, CTAS, RES>, dim3(grid), dim3(256), H * sizeof(float), st, dy, x, w, rstd, dres, dx,
+             dw_acc, rows, H);
+  return grid;
+}
+
+// Which kernel: two or three CTAs per SM, so that one loads while another adds up, where that leaves each six trips or more
+// (fewer are not worth the partial rows) and the scratch has room; a lane then has registers for two or three vectors.
+// Otherwise one CTA per SM with four, and below 1024 rows with two, whose shorter chain of sums at the end counts there.
+// 16384 rows without / with residual, one CTA per SM -> several: of 1024 columns 23.4 / 30.8 -> 21.5 / 27.9 us, of 3072
+// 86.2 / 93.6 -> 59.2 / 68.5, of 4096 without 94.3 -> 77.5 (with: 104.8, several 105.3); 64 rows of 1024 6.0 -> 4.0.
 static int launch_rmsnorm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w, const float* rstd,
                               const __nv_bfloat16* dres, __nv_bfloat16* dx, float* dw_acc, long long rows, int H,
                               int cap, cudaStream_t st) {
-  const int nvec = H / 8;                     // four vectors per lane: with eight the registers do not suffice
-  const int rpc = nvec <= 128 ? 8 : nvec <= 256 ? 4 : nvec <= 512 ? 2 : 1;
-  const long long groups = (rows + rpc - 1) / rpc, trips = (groups + cap - 1) / cap;
-  const int grid = (int)((groups + trips - 1) / trips);
-  auto kern = nvec <= 64 ? rmsnorm_bwd_kernel<2, 1> : nvec <= 128 ? rmsnorm_bwd_kernel<4, 1> :
-              nvec <= 256 ? rmsnorm_bwd_kernel<4, 2> : nvec <= 512 ? rmsnorm_bwd_kernel<4, 4> : rmsnorm_bwd_kernel<4, 8>;
-  launch_pdl(kern, dim3(grid), dim3(256), H * sizeof(float), st, dy, x, w, rstd, dres, dx, dw_acc, rows, H);
-  return grid;
+  const int nvec = H / 8;
+  auto pays = [&](int wpr, int ctas) { return cap >= 148 * ctas && rows * wpr >= 8LL * 6 * 148 * ctas; };
+#define MFSDP_RMS(VPL, WPR, CTAS, CAP)                                                                                    \
+  return dres ? launch_rmsnorm_bwd_as<VPL, WPR, CTAS, true>(dy, x, w, rstd, dres, dx, dw_acc, rows, H, CAP, st)           \
+              : launch_rmsnorm_bwd_as<VPL, WPR, CTAS, false>(dy, x, w, rstd, dres, dx, dw_acc, rows, H, CAP, st)
+  if (nvec <= 64) MFSDP_RMS(2, 1, 2, pays(1, 2) ? 2 * 148 : 148);
+  if (nvec <= 128 && pays(2, 2)) MFSDP_RMS(2, 2, 2, 2 * 148);
+  if (nvec > 128 && nvec <= 192 && pays(2, 2)) MFSDP_RMS(3, 2, 2, 2 * 148);
+  if (nvec > 192 && nvec <= 256 && pays(4, 2)) MFSDP_RMS(2, 4, 2, 2 * 148);
+  if (nvec > 256 && nvec <= 384 && pays(4, 2)) MFSDP_RMS(3, 4, 2, 2 * 148);
+  if (nvec > 384 && nvec <= 512 && !dres && pays(8, 3))
+    return launch_rmsnorm_bwd_as<2, 8, 3, false>(dy, x, w, rstd, dres, dx, dw_acc, rows, H, 3 * 148, st);
+  if (nvec > 512 && nvec <= 768 && pays(8, 2)) MFSDP_RMS(3, 8, 2, 2 * 148);
+  if (nvec <= 128 && rows <= 1024) MFSDP_RMS(2, 2, 2, 148);
+  if (nvec <= 256 && rows <= 1024) MFSDP_RMS(2, 4, 2, 148);
+  if (nvec <= 128) MFSDP_RMS(4, 1, 1, 148);
+  if (nvec <= 256) MFSDP_RMS(4, 2, 1, 148);
+  if (nvec <= 512) MFSDP_RMS(4, 4, 1, 148);
+  MFSDP_RMS(4, 8, 1, 148);
+#undef MFSDP_RMS
 }
 
 // dw_acc: fp32 scratch of mfsdp_rmsnorm_bwd_scratch_rows(rows) x H floats (fully overwritten, needs no

@@ -245,7 +245,7 @@ def rmsnorm_bwd(dy: torch.Tensor, x: torch.Tensor, w: torch.Tensor, rstd: torch.
     x2, dy2 = x.reshape(-1, H), dy.reshape(-1, H)
     assert x2.is_contiguous() and dy2.is_contiguous()
     dx = torch.empty_like(x2)
-    acc = _scratch_f32(min(x2.shape[0], 148) * H, x.device, "rms_dw")
+    acc = _scratch_f32(min(x2.shape[0], 3 * 148) * H, x.device, "rms_dw")      # mfsdp_rmsnorm_bwd_scratch_rows
     if dw_out is None:
         dw_out = torch.empty(H, dtype=torch.bfloat16, device=x.device)
         accumulate_dw = False

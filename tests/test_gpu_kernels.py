@@ -736,3 +736,18 @@ def test_embedding_backward_of_a_frequent_id(K, n, H, accumulate):
     if accumulate:
         total += old.double()
     assert _rel_err(out, total) < 2 ** -8
+
+
+@pytest.mark.parametrize("rows,H", [(14300, 264), (14208, 512), (7105, 520), (7104, 1024), (7110, 1032), (7104, 1536), (3553, 1544),
+                                    (3552, 2048), (3560, 2056), (3552, 3072), (2664, 3080), (2665, 4096), (1777, 4104),
+                                    (1776, 6144), (1030, 6152)])
+def test_rmsnorm_bwd_with_several_blocks_per_sm(K, rows, H):
+    """Row counts from which two or three CTAs share an SM, at both ends of each kernel's widths, and one that keeps a
+    single CTA.  Bounds as in test_rmsnorm_rows_and_widths."""
+    test_rmsnorm_rows_and_widths(K, H, rows)
+
+
+@pytest.mark.parametrize("H", [256, 264, 768, 776, 1544, 3072, 3080, 6144, 6152, 10240, 10248, 14336, 14344])
+def test_rmsnorm_forward_vectors_per_lane(K, H):
+    """Both sides of the widths at which a lane takes one vector more, or a row more warps."""
+    test_rmsnorm_forward_of_the_widest_rows(K, H, 37)
