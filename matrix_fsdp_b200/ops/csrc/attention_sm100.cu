@@ -293,7 +293,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs p
   }
 }
 
-// Forward for grids that fill the chip: one CTA per (batch, head, 256 queries), two 128-query tiles in flight.
+// Forward for grids that fill the chip (attn_fwd_two_tiles): one CTA per (batch, head, 256 queries), two 128-query tiles in flight.
 // One tile's softmax alone leaves the tensor pipe idle while it runs and waits while the pipe works; with two tiles
 // the products of one run beside the softmax of the other.  A thread owns a whole query row (no exchange between
 // threads, no block barrier in the loop) and P goes back to tensor memory over the scores it came from, so it
@@ -900,10 +900,17 @@ static int heads_in_l2(int B, int S, int nH) {
   return (int)(group < 1 ? 1 : group > heads ? heads : group);
 }
 
-// A grid of at most one 128-query tile per SM is as long as its longest tile, which two threads per row finish sooner
-// (16 heads of 1024 rows: 20 us in one-tile blocks, 25 in two); above that two tiles per block win at every size tried.
+// One tile per block: its longest block takes 1.31 us per key tile; two: 1.9 us, for twice the queries (0.72 of the time
+// where the chip is full).  So two tiles lose where the longest block sets the time: while the heads * (nt + 1) / 2 key
+// tiles per query tile, spread over the SMs, leave most of them idle, the more so the longer the rows.  The line is
+// measured (1 to 384 heads of 1 to 128 tiles; one / two tiles per block):
+//   just below it: 2 heads of 128 tiles 170 / 239 us, 4 of 48 68 / 94, 8 of 24 45.7 / 49.9, 16 of 10 23.2 / 24.5
+//   just above:    4 heads of 96 tiles 225 / 186 us, 6 of 48 109 / 98, 8 of 32 74.7 / 68.0, 16 of 12 29.0 / 27.8, 32 of 5 16.8 / 14.6
+// Rows of a single tile have no second one to overlap (192 heads: 11.9 / 12.6).  What the line misses: 96 heads of 3 tiles,
+// 17.4 / 20.2, whose two-tile blocks just begin a second wave.
 static bool attn_fwd_two_tiles(int B, int S, int nH) {
-  return (long long)((S + kBq - 1) / kBq) * nH * B > 148;
+  const long long nt = (S + kBq - 1) / kBq, heads = (long long)nH * B;
+  return nt > 1 && nt * heads > 148 && heads * (nt + 1) > 185 + nt;
 }
 
 // qkv: [B*S, 3*nH*128] bf16 (row stride ld_qkv elements); out: [B*S, nH*128]; lse: [B, nH, S] fp32.

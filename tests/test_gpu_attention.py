@@ -82,8 +82,9 @@ def test_attention_bwd_matches_fp32(B, S, nH):
                                           (2, 255, 40, (1, 39)), (1, 257, 50, (0, 49)), (1, 385, 40, (2, 39)),
                                           (3, 1333, 16, (0, 15)), (1, 8192, 20, (0, 15, 16, 19))])
 def test_attention_fwd_two_tiles_per_block(B, S, nH, heads):
-    """Grids of more than 148 query tiles take the kernel with two of them per block: a lone tile, a second tile of one
-    row, odd and even tile counts, and a last group of heads that is not full.  Bounds as for the other kernel."""
+    """Grids of more than 148 query tiles, which take the kernel with two of them per block from two tiles per row on: a
+    lone tile, a second tile of one row, odd and even tile counts, and a last group of heads that is not full.  Bounds as
+    for the other kernel."""
     from matrix_fsdp_b200.ops import attention as A
     from matrix_fsdp_b200.ops import kernels as K
 
@@ -147,3 +148,25 @@ def test_attention_bwd_tiles_and_head_groups(B, S, nH, heads):
                 # with one row P is 1 and dS cancels: the rounding of dO and O remains, 2^-8 of their products
                 floor = 2 ** -7 * one[:, :].norm() if S == 1 else 0.0
                 assert (g - w).norm() <= 1e-2 * w.norm() + floor, (b, h, i)
+
+
+@pytest.mark.parametrize("B,S,nH,two", [(2, 1000, 10, False), (2, 1000, 11, True), (1, 8100, 3, False), (1, 8100, 4, True),
+                                        (150, 1, 1, False), (2, 129, 38, True)])
+def test_attention_fwd_on_both_sides_of_the_line(B, S, nH, two):
+    """One or two query tiles per block: 185 + tiles key tiles per query tile, more than a wave of tiles, more than one
+    tile per row.  Bounds as for either kernel."""
+    from matrix_fsdp_b200.ops import attention as A
+    from matrix_fsdp_b200.ops import kernels as K
+
+    nt = (S + 127) // 128
+    assert (nt > 1 and nt * B * nH > 148 and B * nH * (nt + 1) > 185 + nt) == two
+    torch.manual_seed(S)
+    hd = 128
+    qkv = torch.randn(B * S, 3 * nH * hd, device="cuda", dtype=torch.bfloat16)
+    out, lse = A.attention_fwd(qkv, B, S, nH, hd)
+    K.check_status()
+    for b, h in ((0, 0), (B - 1, nH - 1)):
+        one = torch.cat([qkv[b * S:(b + 1) * S, (i * nH + h) * hd:(i * nH + h + 1) * hd] for i in range(3)], dim=1)
+        ref_o, ref_lse = _ref(one, 1, S, 1, hd)
+        assert (out[b * S:(b + 1) * S, h * hd:(h + 1) * hd].float() - ref_o).abs().max().item() < 3e-2
+        assert (lse[b, h] - ref_lse[0, 0]).abs().max().item() < 2e-3
