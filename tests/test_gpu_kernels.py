@@ -744,10 +744,10 @@ def test_embedding_backward_of_a_frequent_id(K, n, H, accumulate):
 def test_rmsnorm_bwd_with_several_blocks_per_sm(K, rows, H):
     """Row counts from which two or three CTAs share an SM, at both ends of each kernel's widths, and one that keeps a
     single CTA.  Bounds as in test_rmsnorm_rows_and_widths."""
-    test_rmsnorm_rows_and_widths(K, H, rows)
+    test_rmsnorm_rows_and_widths(K, rows=rows, H=H)
 
 
 @pytest.mark.parametrize("H", [256, 264, 768, 776, 1544, 3072, 3080, 6144, 6152, 10240, 10248, 14336, 14344])
 def test_rmsnorm_forward_vectors_per_lane(K, H):
     """Both sides of the widths at which a lane takes one vector more, or a row more warps."""
-    test_rmsnorm_forward_of_the_widest_rows(K, H, 37)
+    test_rmsnorm_forward_of_the_widest_rows(K, rows=37, H=H)
