@@ -22,8 +22,8 @@
 
 namespace mfsdp {
 
-int make_tmap_bf16_2d(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld,
-                      int box_rows, int box_cols);   // defined in gemm_sm100.cu (cached)
+int make_tmap_bf16(CUtensorMap* map, const void* base, long long batches, long long rows, long long cols, long long ld,
+                   int box_rows, int box_cols);      // defined in gemm_sm100.cu (cached)
 void ensure_context_on_this_thread();                // likewise
 
 constexpr int kHd = 128;            // head dim
@@ -80,10 +80,12 @@ __device__ __forceinline__ void mma_tile_128(uint32_t tmem_d, uint32_t a_base, b
   }
 }
 
-// Load a [128 rows x 128 cols] bf16 tile whose top-left corner is (row0, col0) as two 64-column boxes.
-__device__ __forceinline__ void tma_load_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, int col0, int row0) {
-  tma_load_2d(dst, map, bar, col0, row0);
-  tma_load_2d(dst + kHalfTile, map, bar, col0 + 64, row0);
+// Load a [128 rows x 128 cols] bf16 tile of one sequence, whose top-left corner is (row0, col0), as two 64-column boxes.
+// Rows past the end of the sequence are zeros and cost no traffic (they are not the next sequence's: its values, infinities
+// among them, have no way into this one's products).
+__device__ __forceinline__ void tma_load_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, int col0, int row0, int batch) {
+  tma_load_3d(dst, map, bar, col0, row0, batch);
+  tma_load_3d(dst + kHalfTile, map, bar, col0 + 64, row0, batch);
 }
 
 __global__ void __launch_bounds__(kAttnThreads, 1)
@@ -134,15 +136,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs p
   if (warp == 0) {
     if (lane == 0) {
       mbar_arrive_expect_tx(smem_u32(q_full), kTileBytes);
-      tma_load_tile(sQ, &tma_qkv, smem_u32(q_full), h * kHd, row_base + q0);
+      tma_load_tile(sQ, &tma_qkv, smem_u32(q_full), h * kHd, q0, b);
       for (int j = 0; j < nkv; ++j) {
         const uint32_t s = j & 1, ph = (j >> 1) & 1;
         if (!mbar_wait(smem_u32(&k_empty[s]), ph ^ 1, p.status, abort_flag)) break;
         mbar_arrive_expect_tx(smem_u32(&k_full[s]), kTileBytes);
-        tma_load_tile(sK + s * kTileBytes, &tma_qkv, smem_u32(&k_full[s]), H + h * kHd, row_base + j * kBk);
+        tma_load_tile(sK + s * kTileBytes, &tma_qkv, smem_u32(&k_full[s]), H + h * kHd, j * kBk, b);
         if (!mbar_wait(smem_u32(&v_empty[s]), ph ^ 1, p.status, abort_flag)) break;
         mbar_arrive_expect_tx(smem_u32(&v_full[s]), kTileBytes);
-        tma_load_tile(sV + s * kTileBytes, &tma_qkv, smem_u32(&v_full[s]), 2 * H + h * kHd, row_base + j * kBk);
+        tma_load_tile(sV + s * kTileBytes, &tma_qkv, smem_u32(&v_full[s]), 2 * H + h * kHd, j * kBk, b);
       }
     }
   } else if (warp == 1) {
@@ -379,16 +381,16 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs 
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
     if (warp == 0 && lane == 0) {
       mbar_arrive_expect_tx(smem_u32(q_full), n1 > 0 ? 2 * kTileBytes : kTileBytes);
-      tma_load_tile(sQ, &tma_qkv, smem_u32(q_full), h * kHd, row_base + q0);
-      if (n1 > 0) tma_load_tile(sQ + kTileBytes, &tma_qkv, smem_u32(q_full), h * kHd, row_base + q0 + kBq);
+      tma_load_tile(sQ, &tma_qkv, smem_u32(q_full), h * kHd, q0, b);
+      if (n1 > 0) tma_load_tile(sQ + kTileBytes, &tma_qkv, smem_u32(q_full), h * kHd, q0 + kBq, b);
       for (int j = 0; j < n_max; ++j) {
         const uint32_t s = j & 1, ph = (j >> 1) & 1;
         if (!mbar_wait(smem_u32(&k_empty[s]), ph ^ 1, p.status, abort_flag)) break;
         mbar_arrive_expect_tx(smem_u32(&k_full[s]), kTileBytes);
-        tma_load_tile(sK + s * kTileBytes, &tma_qkv, smem_u32(&k_full[s]), H + h * kHd, row_base + j * kBk);
+        tma_load_tile(sK + s * kTileBytes, &tma_qkv, smem_u32(&k_full[s]), H + h * kHd, j * kBk, b);
         if (!mbar_wait(smem_u32(&v_empty[s]), ph ^ 1, p.status, abort_flag)) break;
         mbar_arrive_expect_tx(smem_u32(&v_full[s]), kTileBytes);
-        tma_load_tile(sV + s * kTileBytes, &tma_qkv, smem_u32(&v_full[s]), 2 * H + h * kHd, row_base + j * kBk);
+        tma_load_tile(sV + s * kTileBytes, &tma_qkv, smem_u32(&v_full[s]), 2 * H + h * kHd, j * kBk, b);
       }
     } else if (warp == 1 && lane == 0) {
       constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
@@ -664,25 +666,25 @@ __device__ __forceinline__ void attn_bwd_block(const CUtensorMap& tma_qkv, const
     if (warp == 0 && lane == 0) {
       mbar_arrive_expect_tx(smem_u32(stat_full), 2 * kTileBytes);
       if (DQ) {
-        tma_load_tile(sA0, &tma_qkv, smem_u32(stat_full), h * kHd, row_base + r0);          // Q_i
-        tma_load_tile(sA1, &tma_do, smem_u32(stat_full), h * kHd, row_base + r0);           // dO_i
+        tma_load_tile(sA0, &tma_qkv, smem_u32(stat_full), h * kHd, r0, b);          // Q_i
+        tma_load_tile(sA1, &tma_do, smem_u32(stat_full), h * kHd, r0, b);           // dO_i
       } else {
-        tma_load_tile(sA0, &tma_qkv, smem_u32(stat_full), H + h * kHd, row_base + r0);      // K_j
-        tma_load_tile(sA1, &tma_qkv, smem_u32(stat_full), 2 * H + h * kHd, row_base + r0);  // V_j
+        tma_load_tile(sA0, &tma_qkv, smem_u32(stat_full), H + h * kHd, r0, b);      // K_j
+        tma_load_tile(sA1, &tma_qkv, smem_u32(stat_full), 2 * H + h * kHd, r0, b);  // V_j
       }
       for (int k = 0; k < 2 * T; ++k) {
         if (!mbar_wait(smem_u32(&empty[k % kRing]), full_phase(k) ^ 1, p.status, abort_flag)) break;
         const uint32_t bar = full_bar(k);
         mbar_arrive_expect_tx(bar, kTileBytes + (DQ ? 0 : kStatBytes));
-        const int i = k >> 1, t0 = (t_begin + i) * 128, row = row_base + t0;
+        const int i = k >> 1, t0 = (t_begin + i) * 128;
         const long long stat = (long long)bh * p.Sp + t0;
         if (DQ) {
-          tma_load_tile(slot(k), &tma_qkv, bar, ((k & 1) ? 2 * H : H) + h * kHd, row);          // K_t, V_t
+          tma_load_tile(slot(k), &tma_qkv, bar, ((k & 1) ? 2 * H : H) + h * kHd, t0, b);          // K_t, V_t
         } else if (k & 1) {
-          tma_load_tile(slot(k), &tma_do, bar, h * kHd, row);                                   // dO_t
+          tma_load_tile(slot(k), &tma_do, bar, h * kHd, t0, b);                                   // dO_t
           bulk_load(smem_u32(smem + AttnBwdSmem::kNdelta + (i & 1) * kStatBytes), p.ndelta + stat, kStatBytes, bar);
         } else {
-          tma_load_tile(slot(k), &tma_qkv, bar, h * kHd, row);                                  // Q_t
+          tma_load_tile(slot(k), &tma_qkv, bar, h * kHd, t0, b);                                  // Q_t
           bulk_load(smem_u32(smem + AttnBwdSmem::kNlse + (i % 3) * kStatBytes), p.nlse2 + stat, kStatBytes, bar);
         }
       }
@@ -919,7 +921,7 @@ MFSDP_API int mfsdp_attention_fwd(const void* qkv, void* out, float* lse, int B,
   if (B <= 0 || S <= 0 || nH <= 0 || (ld_qkv % 8) || (ld_out % 8)) return -2;
   ensure_context_on_this_thread();
   CUtensorMap map;
-  int rc = make_tmap_bf16_2d(&map, qkv, (long long)B * S, 3LL * nH * kHd, ld_qkv, 128, 64);
+  int rc = make_tmap_bf16(&map, qkv, B, S, 3LL * nH * kHd, ld_qkv, 128, 64);
   if (rc) return rc;
   static bool attr = false;
   if (!attr) {
@@ -950,9 +952,9 @@ MFSDP_API int mfsdp_attention_bwd(const void* dout, const void* qkv, const void*
   if (B <= 0 || S <= 0 || nH <= 0 || (ld_qkv % 8) || (ld_o % 8) || (ld_dqkv % 8) || !scratch || ((uintptr_t)scratch & 15)) return -2;
   ensure_context_on_this_thread();
   CUtensorMap map_qkv, map_do;
-  int rc = make_tmap_bf16_2d(&map_qkv, qkv, (long long)B * S, 3LL * nH * kHd, ld_qkv, 128, 64);
+  int rc = make_tmap_bf16(&map_qkv, qkv, B, S, 3LL * nH * kHd, ld_qkv, 128, 64);
   if (rc) return rc;
-  rc = make_tmap_bf16_2d(&map_do, dout, (long long)B * S, (long long)nH * kHd, ld_o, 128, 64);
+  rc = make_tmap_bf16(&map_do, dout, B, S, (long long)nH * kHd, ld_o, 128, 64);
   if (rc) return rc;
   static bool attr = false;
   if (!attr) {

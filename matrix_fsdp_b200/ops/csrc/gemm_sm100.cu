@@ -549,10 +549,10 @@ static EncodeTiledFn get_encode_fn() {
 // activation buffers), so encoded maps are kept in a small per-process table.
 struct TmapKey {
   const void* base;
-  long long rows, cols, ld;
+  long long batches, rows, cols, ld;       // batches = 0: two dimensions
   int box_rows, box_cols;
   bool operator==(const TmapKey& o) const {
-    return base == o.base && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows &&
+    return base == o.base && batches == o.batches && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows &&
            box_cols == o.box_cols;
   }
 };
@@ -584,9 +584,11 @@ void ensure_context_on_this_thread() {
 }
 
 // rows x cols row-major bf16 tensor (row stride `ld` elements); box = box_rows x box_cols.
-int make_tmap_bf16_2d(CUtensorMap* map, const void* base, long long rows, long long cols,
-                      long long ld, int box_rows, int box_cols) {
-  const TmapKey key{base, rows, cols, ld, box_rows, box_cols};
+// Tensor map of a row-major bf16 matrix (batches = 0), or of `batches` matrices of `rows` rows one behind the other with a
+// batch coordinate of their own: a box that reaches past a matrix' last row is then filled with zeros.
+int make_tmap_bf16(CUtensorMap* map, const void* base, long long batches, long long rows, long long cols, long long ld,
+                   int box_rows, int box_cols) {
+  const TmapKey key{base, batches, rows, cols, ld, box_rows, box_cols};
   TmapSlot& slot = g_tmap_cache[tmap_hash(key)];
   {
     std::lock_guard<std::mutex> lock(g_tmap_mutex);
@@ -598,11 +600,11 @@ int make_tmap_bf16_2d(CUtensorMap* map, const void* base, long long rows, long l
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return -1;
   ensure_context_on_this_thread();
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides,
+  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batches};
+  cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)(rows * ld) * 2};
+  cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, batches > 0 ? 3 : 2, const_cast<void*>(base), dims, strides,
                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return (int)r;
@@ -611,6 +613,11 @@ int make_tmap_bf16_2d(CUtensorMap* map, const void* base, long long rows, long l
   slot.map = *map;
   slot.used = true;
   return 0;
+}
+
+static int make_tmap_bf16_2d(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_rows,
+                             int box_cols) {
+  return make_tmap_bf16(map, base, 0, rows, cols, ld, box_rows, box_cols);
 }
 
 template <int BN, bool A_MN, bool B_MN, bool GATHER, bool ADD_C>

@@ -170,3 +170,25 @@ def test_attention_fwd_on_both_sides_of_the_line(B, S, nH, two):
         ref_o, ref_lse = _ref(one, 1, S, 1, hd)
         assert (out[b * S:(b + 1) * S, h * hd:(h + 1) * hd].float() - ref_o).abs().max().item() < 3e-2
         assert (lse[b, h] - ref_lse[0, 0]).abs().max().item() < 2e-3
+
+
+@pytest.mark.parametrize("B,S,nH", [(3, 200, 2), (5, 64, 16), (2, 1000, 11), (4, 129, 40)])
+def test_sequences_do_not_reach_into_each_other(B, S, nH):
+    """Infinities and NaN in the other sequences of a batch leave the first one's results as they are, bit for bit, although
+    its last tile ends behind its last row (one tile per block and two, both directions)."""
+    from matrix_fsdp_b200.ops import attention as A
+    from matrix_fsdp_b200.ops import kernels as K
+
+    torch.manual_seed(S)
+    hd = 128
+    qkv = torch.randn(B * S, 3 * nH * hd, device="cuda", dtype=torch.bfloat16)
+    dout = torch.randn(B * S, nH * hd, device="cuda", dtype=torch.bfloat16)
+
+    def first():
+        out, lse = A.attention_fwd(qkv, B, S, nH, hd)
+        return out[:S], lse[0], A.attention_bwd(dout, qkv, out, lse, B, S, nH, hd)[:S]
+
+    want = first()
+    qkv[S:], dout[S:] = math.inf, math.nan
+    assert all(torch.equal(a, b) for a, b in zip(first(), want))
+    K.check_status()
