@@ -557,8 +557,9 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tma_qkv, const AttnFwdArgs 
 // arrive with it, in the same barriers, so no thread waits for another.
 // Four threads share a row: with two (2 warps per scheduler) the fixed latencies of the element-wise chains showed.
 // Measured (64-wide streamed tiles -> 128-wide in pairs of buffers -> this): 16 heads of 2 x 4096 rows 806 -> 547 ->
-// 503 us, 32 heads of 16384 rows 10.1 -> 7.2 -> 6.4 ms (857 TFLOP/s counting five products per tile), 16 heads of
-// 3 x 1333 rows 205 -> 157 -> 152 us.
+// 492 us, 16 heads of 3 x 1333 rows 201 -> 157 -> 135 us; 32 heads of 16384 rows 9.9 -> 7.2 -> 6.9 to 7.4 ms back to back,
+// where the power cap takes the clock to 1.69 GHz, and 6.6 ms (838 TFLOP/s counting five products per tile) in calls
+// apart from one another.
 constexpr int kBwdThreads = 640;      // warp 0 TMA, warp 1 MMA, 2 and 3 idle, warps 4-19 P and dS
 constexpr int kBwdCols = 32;          // streamed columns per thread
 // 640 threads are launched with 96 registers each, 61,440 in all: 128 * 64 + 512 * 104.
@@ -600,7 +601,7 @@ __device__ __forceinline__ void mma_acc_ts(uint32_t tmem_d, uint32_t tmem_p, uin
   }
 }
 
-template <bool DQ>
+template <bool DQ, bool SKIP>
 __device__ __forceinline__ void attn_bwd_block(const CUtensorMap& tma_qkv, const CUtensorMap& tma_do, const AttnBwdArgs& p,
                                                const int block) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -764,8 +765,14 @@ __device__ __forceinline__ void attn_bwd_block(const CUtensorMap& tma_qkv, const
       const bool need_mask = c0 == r0 || (!DQ && c0 + 128 > p.S);
       const uint64_t* nlse = reinterpret_cast<const uint64_t*>(smem + AttnBwdSmem::kNlse + (i % 3) * kStatBytes) + part * (kBwdCols / 2);
       const uint64_t* ndelta = reinterpret_cast<const uint64_t*>(smem + AttnBwdSmem::kNdelta + (i & 1) * kStatBytes) + part * (kBwdCols / 2);
+      // a warp none of whose elements counts writes its zeros without computing them
+      const int e0 = c0 + part * kBwdCols, w0 = r0 + q * 32;
+      const bool skip = SKIP && need_mask && (w0 >= p.S || (DQ ? e0 > w0 + 31 : (e0 + kBwdCols <= w0 || e0 >= p.S)));
       float pe[kBwdCols];
-      {
+      if (skip) {
+#pragma unroll
+        for (int e = 0; e < kBwdCols; ++e) pe[e] = 0.f;
+      } else {
         uint32_t sv[kBwdCols];
         tmem_ld_32x32b_x32(my_s, sv);
         tmem_ld_wait();
@@ -776,7 +783,7 @@ __device__ __forceinline__ void attn_bwd_block(const CUtensorMap& tma_qkv, const
           pe[2 * e + 1] = exp2f(pe[2 * e + 1]);
         }
       }
-      if (need_mask) mask_row(pe, c0 + part * kBwdCols);
+      if (need_mask && !skip) mask_row(pe, e0);
       if (!DQ) {
         uint32_t pk[kBwdCols / 2];
 #pragma unroll
@@ -790,7 +797,13 @@ __device__ __forceinline__ void attn_bwd_block(const CUtensorMap& tma_qkv, const
       mbar_arrive(smem_u32(p_ready));
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(dp_full), i & 1, p.status, abort_flag))) { ok = false; break; }
       tc_fence_after();
-      {
+      if (skip) {
+        uint32_t pk[kBwdCols / 2];
+#pragma unroll
+        for (int e = 0; e < kBwdCols / 2; ++e) pk[e] = 0u;
+        tmem_st_32x32b_x16(my_dp, pk);
+        tmem_st_wait();
+      } else {
         uint32_t dv[kBwdCols], pk[kBwdCols / 2];
         tmem_ld_32x32b_x32(my_dp, dv);
         tmem_ld_wait();
@@ -799,7 +812,7 @@ __device__ __forceinline__ void attn_bwd_block(const CUtensorMap& tma_qkv, const
           unpack_f32x2(mul_f32x2(pack_f32x2(pe[2 * e], pe[2 * e + 1]),
                                  add_f32x2(pack_u32x2(dv[2 * e], dv[2 * e + 1]), DQ ? own_ndelta : ndelta[e])),
                        pe[2 * e], pe[2 * e + 1]);
-        if (need_mask) mask_row(pe, c0 + part * kBwdCols);         // 0 * inf from elements that do not count
+        if (need_mask) mask_row(pe, e0);         // 0 * inf from elements that do not count
 #pragma unroll
         for (int e = 0; e < kBwdCols / 2; ++e) pk[e] = pack_bf16x2(pe[2 * e], pe[2 * e + 1]);
         tmem_st_32x32b_x16(my_dp, pk);
@@ -849,12 +862,13 @@ __device__ __forceinline__ void attn_bwd_block(const CUtensorMap& tma_qkv, const
 // second (a head of 1024 rows has 8 blocks of each kind, 1 to 8 tiles long).  Two launches -> one, preparation included:
 // 16 heads of 1024 rows 51.5 -> 36.6 us, of 4 x 1024 132 -> 120 us, of 3 x 1333 155 -> 143 us, 8 heads of 8192 rows 478 ->
 // 441 us.  Alternating kinds were slower at long rows, where each streams tensors of its own through the L2.
+template <bool SKIP>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_qkv, const __grid_constant__ CUtensorMap tma_do,
                 const __grid_constant__ AttnBwdArgs p) {
   const int n = (int)(gridDim.x >> 1), block = (int)blockIdx.x;
-  if (block < n) attn_bwd_block<false>(tma_qkv, tma_do, p, block);
-  else attn_bwd_block<true>(tma_qkv, tma_do, p, block - n);
+  if (block < n) attn_bwd_block<false, SKIP>(tma_qkv, tma_do, p, block);
+  else attn_bwd_block<true, SKIP>(tma_qkv, tma_do, p, block - n);
 }
 
 // nlse2 = -lse * log2(e); ndelta = -rowsum(dO * O); both zero for the rows that pad a head to whole tiles.  Half a
@@ -956,9 +970,15 @@ MFSDP_API int mfsdp_attention_bwd(const void* dout, const void* qkv, const void*
   if (rc) return rc;
   rc = make_tmap_bf16(&map_do, dout, B, S, (long long)nH * kHd, ld_o, 128, 64);
   if (rc) return rc;
+  // Rows of up to a few tiles consist of tiles on the diagonal and at the end, most of whose 32 x 32 parts do not count:
+  // leaving those out takes 512 heads of 32 rows from 48.9 to 43.5 us, 256 of 64 30.9 to 28.6, 128 of 300 58.8 to 56.2, 48 of
+  // 777 70.8 to 69.2.  From about 1024 rows on whole tiles prevail and lose by it (32 heads of 4096 rows 492 / 504 us).
+  const auto kern = S < 1024 ? attn_bwd_kernel<true> : attn_bwd_kernel<false>;
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnBwdSmem::kBytes);
+    cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnBwdSmem::kBytes);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(attn_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnBwdSmem::kBytes);
     if (e != cudaSuccess) return (int)e;
     attr = true;
   }
@@ -975,6 +995,6 @@ MFSDP_API int mfsdp_attention_bwd(const void* dout, const void* qkv, const void*
   a.nlse2 = nlse2; a.ndelta = ndelta;
   a.dqkv = (__nv_bfloat16*)dqkv; a.ld_dqkv = ld_dqkv; a.status = status;
   a.heads_per_group = heads_in_l2(B, S, nH);
-  return launch_pdl(attn_bwd_kernel, dim3(2u * (unsigned)(nt * B * nH)), dim3(kBwdThreads), AttnBwdSmem::kBytes, st, map_qkv,
+  return launch_pdl(kern, dim3(2u * (unsigned)(nt * B * nH)), dim3(kBwdThreads), AttnBwdSmem::kBytes, st, map_qkv,
                     map_do, a);
 }

@@ -192,3 +192,10 @@ def test_sequences_do_not_reach_into_each_other(B, S, nH):
     qkv[S:], dout[S:] = math.inf, math.nan
     assert all(torch.equal(a, b) for a, b in zip(first(), want))
     K.check_status()
+
+
+@pytest.mark.parametrize("S", [31, 32, 33, 64, 65, 97, 161, 1023, 1024])
+def test_attention_bwd_parts_that_do_not_count(S):
+    """Rows short enough that whole 32 x 32 parts of a tile are left out: both sides of a part's edge, and of the row count
+    from which they are computed and masked.  Bound as for the other sizes."""
+    test_attention_bwd_tiles_and_head_groups(B=2, S=S, nH=3, heads=(0, 2))
