@@ -146,7 +146,11 @@ class _EmbeddingFn(torch.autograd.Function):
         return None, dw, None
 
 
-_EMBED_MAX_TOKENS = 32768       # the rank pass compares every position with the earlier ones
+# Uniform ids are summed four to nine times faster than by the library (4096 positions, 32000 ids, 1024 columns: 46 against
+# 214 us; 32768: 73 against 659; 65536: 93 against 801), but one block adds up all rows of one id, which the library
+# splits: half of the positions the same (padding) take 1.8 against 0.6 ms at 32768 positions and 3.6 against 0.8 at 65536.
+# The limit bounds that loss.
+_EMBED_MAX_TOKENS = 32768
 
 
 def embedding(ids: torch.Tensor, weight: torch.Tensor, param: torch.nn.Parameter | None = None) -> torch.Tensor:
