@@ -481,7 +481,19 @@ __device__ __forceinline__ float ieee_fma(float a, float b, float c) { float d; 
 __device__ __forceinline__ float ieee_div(float a, float b) { float d; asm("div.rn.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b)); return d; }
 __device__ __forceinline__ float ieee_sqrt(float a) { float d; asm("sqrt.rn.f32 %0, %1;" : "=f"(d) : "f"(a)); return d; }
 
+// EXACT: as torch's operations round.  Otherwise approximate quotients and root (a few units in the last place of a step):
+// the updates of units run beside the backward's GEMMs, and the instructions of the exact ones cost a training step of 8
+// layers of 2048 1.4 % (14.87 -> 15.09 ms).
+template <bool EXACT>
 __device__ __forceinline__ void adamw_update(float& p, float& m, float& v, float g, const AdamWStep& a) {
+  if (!EXACT) {
+    g *= a.grad_scale;
+    p *= a.keep;
+    m = a.beta1 * m + a.one_minus_beta1 * g;
+    v = a.beta2 * v + a.one_minus_beta2 * g * g;
+    p -= a.step_size * (m / (sqrtf(v) / a.bias2_sqrt + a.eps));
+    return;
+  }
   g = ieee_mul(g, a.grad_scale);
   // between m and g from the nearer end, as torch's lerp: one rounded constant instead of two that do not add up to one
   const float d = ieee_add(g, -m);

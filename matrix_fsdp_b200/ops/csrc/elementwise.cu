@@ -402,11 +402,10 @@ cross_entropy_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const long long
 // on the fly; the kernel also emits the low-precision copy that the next all-gather
 // ships, so no separate cast kernel runs.  Matches torch.optim.AdamW (decoupled decay,
 // bias correction, eps outside the sqrt of the corrected second moment).
-// Bound by memory.  Four blocks per SM: with the 72 registers that the compiler takes for the correctly rounded operations
-// when it is free to, too few loads are in flight (50 M parameters, bf16 gradients: 246 us; four blocks 229, 6.1 TB/s;
-// with fast-math operators, in 40 registers, 239).
-template <typename GradT>
-__global__ void __launch_bounds__(256, 4) adamw_flat_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
+// Bound by memory: 50 M parameters, bf16 gradients 239 us (5.9 TB/s).  EXACT: four blocks per SM, because with the 72
+// registers that the compiler takes for it when it is free to too few loads are in flight (246 us; four blocks 229).
+template <typename GradT, bool EXACT>
+__global__ void __launch_bounds__(256, EXACT ? 4 : 6) adamw_flat_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
                                   const GradT* __restrict__ g, __nv_bfloat16* __restrict__ p_lp,
                                   long long n, const AdamWStep a) {
   const long long nv = n >> 2;
@@ -428,7 +427,7 @@ __global__ void __launch_bounds__(256, 4) adamw_flat_kernel(float* __restrict__ 
     float* ma = reinterpret_cast<float*>(&mm);
     float* va = reinterpret_cast<float*>(&vv);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) adamw_update(pa[e], ma[e], va[e], gg[e], a);
+    for (int e = 0; e < 4; ++e) adamw_update<EXACT>(pa[e], ma[e], va[e], gg[e], a);
     reinterpret_cast<float4*>(p)[i] = pp;
     reinterpret_cast<float4*>(m)[i] = mm;
     reinterpret_cast<float4*>(v)[i] = vv;
@@ -441,7 +440,7 @@ __global__ void __launch_bounds__(256, 4) adamw_flat_kernel(float* __restrict__ 
     if constexpr (sizeof(GradT) == 2) gr = __bfloat162float(g[i]);
     else gr = (float)g[i];
     float pv = p[i], mv = m[i], vv = v[i];
-    adamw_update(pv, mv, vv, gr, a);
+    adamw_update<EXACT>(pv, mv, vv, gr, a);
     p[i] = pv; m[i] = mv; v[i] = vv;
     if (p_lp) p_lp[i] = __float2bfloat16_rn(pv);
   }
@@ -1094,17 +1093,17 @@ MFSDP_API int mfsdp_cross_entropy_dev_scale(void* logits, const long long* targe
 
 MFSDP_API int mfsdp_adamw_flat(float* p, float* m, float* v, const void* g, int grad_is_bf16, void* p_lp,
                                long long n, double lr, double beta1, double beta2, double eps,
-                               double weight_decay, long long step, double grad_scale, cudaStream_t st) {
+                               double weight_decay, long long step, double grad_scale, int exact, cudaStream_t st) {
   if (n <= 0) return 0;
   if (((uintptr_t)p & 15) || ((uintptr_t)m & 15) || ((uintptr_t)v & 15) ||
       ((uintptr_t)g & (grad_is_bf16 ? 7 : 15)) || ((uintptr_t)p_lp & 7))
     return -2;
   const AdamWStep a = adamw_step(lr, beta1, beta2, eps, weight_decay, step, grad_scale);
   const int grid = grid_for(n / 4 + 1, 256, 148 * 8);
-  if (grad_is_bf16)
-    adamw_flat_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p, m, v, (const __nv_bfloat16*)g, (__nv_bfloat16*)p_lp, n, a);
-  else
-    adamw_flat_kernel<float><<<grid, 256, 0, st>>>(p, m, v, (const float*)g, (__nv_bfloat16*)p_lp, n, a);
+  auto kern_bf16 = exact ? adamw_flat_kernel<__nv_bfloat16, true> : adamw_flat_kernel<__nv_bfloat16, false>;
+  auto kern_fp32 = exact ? adamw_flat_kernel<float, true> : adamw_flat_kernel<float, false>;
+  if (grad_is_bf16) kern_bf16<<<grid, 256, 0, st>>>(p, m, v, (const __nv_bfloat16*)g, (__nv_bfloat16*)p_lp, n, a);
+  else kern_fp32<<<grid, 256, 0, st>>>(p, m, v, (const float*)g, (__nv_bfloat16*)p_lp, n, a);
   return (int)cudaGetLastError();
 }
 

@@ -302,7 +302,7 @@ __global__ void rs_pull_adamw_kernel(PeerPtrs grads, int world_rt, int rank, Red
       load8(a.m + j, mm);
       load8(a.v + j, vv);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) adamw_update(pp[e], mm[e], vv[e], acc[e] * scale, a.step);
+      for (int e = 0; e < 8; ++e) adamw_update<false>(pp[e], mm[e], vv[e], acc[e] * scale, a.step);
       store8(a.p + j, pp);
       store8(a.m + j, mm);
       store8(a.v + j, vv);
@@ -316,7 +316,7 @@ __global__ void rs_pull_adamw_kernel(PeerPtrs grads, int world_rt, int rank, Red
       }
       const long long j = l0 + i;
       float pp = a.p[j], mm = a.m[j], vv = a.v[j];
-      adamw_update(pp, mm, vv, acc * scale, a.step);
+      adamw_update<false>(pp, mm, vv, acc * scale, a.step);
       a.p[j] = pp; a.m[j] = mm; a.v[j] = vv;
       if (a.p_lp) a.p_lp[j] = __float2bfloat16_rn(pp);
     }
@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(256, 2) rs_mc_adamw_kernel(const TIn* mc_grad,
         load8(a.m + j, mm);
         load8(a.v + j, vv);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) adamw_update(pp[e], mm[e], vv[e], acc[e] * scale, a.step);
+        for (int e = 0; e < 8; ++e) adamw_update<false>(pp[e], mm[e], vv[e], acc[e] * scale, a.step);
         store8(a.p + j, pp);
         store8(a.m + j, mm);
         store8(a.v + j, vv);

@@ -331,13 +331,14 @@ def cross_entropy_(logits: torch.Tensor, target: torch.Tensor, grad_scale: float
 # ------------------------------------------------------------------ optimizers
 def adamw_flat_(p: torch.Tensor, m: torch.Tensor, v: torch.Tensor, g: torch.Tensor, *, lr: float,
                 beta1: float, beta2: float, eps: float, weight_decay: float, step: int,
-                grad_scale: float = 1.0, p_lp: torch.Tensor | None = None) -> None:
+                grad_scale: float = 1.0, p_lp: torch.Tensor | None = None, exact: bool = False) -> None:
+    """One AdamW step in place.  ``exact``: square root and quotients rounded as torch's fp32 operations round them."""
     assert p.dtype == torch.float32 and m.dtype == torch.float32 and v.dtype == torch.float32
     assert g.dtype in (torch.bfloat16, torch.float32) and g.numel() == p.numel()
     _lib.check(_L().mfsdp_adamw_flat(p.data_ptr(), m.data_ptr(), v.data_ptr(), g.data_ptr(),
                                      int(g.dtype == torch.bfloat16),
                                      p_lp.data_ptr() if p_lp is not None else None, p.numel(),
-                                     lr, beta1, beta2, eps, weight_decay, int(step), grad_scale,
+                                     lr, beta1, beta2, eps, weight_decay, int(step), grad_scale, int(exact),
                                      _stream()), "adamw_flat")
 
 

@@ -34,7 +34,7 @@ _SIGNATURES: dict[str, list] = {
     "mfsdp_embedding_bwd": [vp, i64, vp, vp, i64, i32, i32, i32, i32, vp, vp],
     "mfsdp_cross_entropy": [vp, vp, vp, i64, i32, i64, f32, i64, vp],
     "mfsdp_cross_entropy_dev_scale": [vp, vp, vp, i64, i32, i64, vp, i64, vp],
-    "mfsdp_adamw_flat": [vp, vp, vp, vp, i32, vp, i64, f64, f64, f64, f64, f64, i64, f64, vp],
+    "mfsdp_adamw_flat": [vp, vp, vp, vp, i32, vp, i64, f64, f64, f64, f64, f64, i64, f64, i32, vp],
     "mfsdp_sgd_flat": [vp, vp, vp, i32, vp, i64, f32, f32, f32, f32, i32, vp],
     "mfsdp_muon_momentum": [vp, vp, i32, vp, vp, i64, f32, f32, i32, vp],
     "mfsdp_muon_normalize": [vp, vp, i64, f32, vp],

@@ -252,7 +252,7 @@ class FlatShardedAdamW(_FlatShardedBase):
                         lp = None
                     kernels.adamw_flat_(p.data, st["exp_avg"], st["exp_avg_sq"], p.grad, lr=float(group["lr"]), beta1=b1,
                                         beta2=b2, eps=group["eps"], weight_decay=group["weight_decay"], step=step,
-                                        grad_scale=float(self.grad_scale), p_lp=lp)
+                                        grad_scale=float(self.grad_scale), p_lp=lp, exact=True)
                     if lp is not None:
                         torch.autograd.graph.increment_version(lp)      # as the ``copy_`` of the other path does
                         self.lp_written.add(id(p))

@@ -572,8 +572,9 @@ def _adamw_64(p, m, v, g, step, lr, beta1, beta2, eps, weight_decay):
 @pytest.mark.parametrize("first", [1, 1000])
 def test_adamw_constants_and_rounding(K, route, betas, first):
     """Three steps from step ``first`` against 64 bits, on each way into the update.  Moments: a handful of fp32 roundings
-    a step (the smallest ones, below the normal range, to two units of their spacing); the distance covered by the
-    parameter: the same, plus 2.5 * 2^-24 of the parameter itself per step (decay factor, its product, the sum)."""
+    a step (the smallest ones, below the normal range, to two units of their spacing outside units; the other kernels
+    flush them); the distance covered by the parameter: the same (approximate root and quotients: 4 units in the last
+    place more), plus 2.5 * 2^-24 of the parameter itself per step (decay factor, its product, the sum)."""
     import ctypes as C
 
     from matrix_fsdp_b200.ops import lib
@@ -609,7 +610,8 @@ def test_adamw_constants_and_rounding(K, route, betas, first):
         _adamw_64(*want, p.grad.double(), step, beta1=betas[0], beta2=betas[1], **hp)
     K.check_status()
     assert ((m.double() - want[1]).abs() <= 1e-6 * want[1].abs() + 3 * 2 ** -24 * 3e-3).all()
-    assert ((v.double() - want[2]).abs() <= 1e-6 * want[2] + 6 * 2 ** -149).all()
+    tiny = 6 * 2 ** -149 if route == "outside units" else 3 * 2 ** -126
+    assert ((v.double() - want[2]).abs() <= 1e-6 * want[2] + tiny).all()
     moved = (want[0] - p0.double()).abs()
     assert ((p.detach().double() - want[0]).abs() <= 2e-6 * moved + 4 * 2 ** -23 * p0.double().abs().clamp_min(2 ** -8)).all()
 
